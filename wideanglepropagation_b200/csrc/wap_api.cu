@@ -95,26 +95,6 @@ size_t col_smem_bytes(int w, int extra_bytes) {
   return (size_t)N * w * sizeof(float2) + FFTPlan<N, E>::TW_SIZE * sizeof(float4) + extra_bytes;
 }
 
-// Row and column passes go out with programmatic dependent launch (the
-// kernels wait for their predecessor first thing): in a chain of short,
-// latency-bound passes the next pass is already resident when one finishes
-// (C1 0.26 -> 0.19 ms per call).  The WPM passes launch normally: their large
-// CTAs parked early cost more than the launch latency saved (C3 12.5 vs 13.1 ms).
-template <class K, class A>
-static cudaError_t launch_pdl(K kern, dim3 grid, int threads, size_t smem, cudaStream_t st, const A& args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, args);
-}
-
 template <int N, int E>
 static cudaError_t launch_row_t(const RowArgs& a, int nb, int rows, cudaStream_t st) {
   const size_t smem = row_smem_bytes<N, E>(rows, 0);
@@ -345,6 +325,9 @@ static void plan_free(wap_plan* p) {
   cudaFree(p->ky2);
   cudaFree(p->kx2);
   cudaFree(p->refs);
+  cudaFree(p->slices);
+  cudaFree(p->wn_tw_row);
+  cudaFree(p->wn_tw_col);
   cudaFree(p->ttab);
   cudaFree(p->counter);
   cudaFree(p->chain_tw);
@@ -409,6 +392,10 @@ int wap_plan_create(wap_plan** out, int ny, int nx, int max_batch, int op, int n
     if (err != cudaSuccess) {
       plan_free(p);
       return cuda_fail(err, "cudaMalloc(WPM workspace)");
+    }
+    if (!generic && (rc = wpm_node_twiddles(p)) != WAP_OK) {
+      plan_free(p);
+      return rc;
     }
   }
   *out = p;

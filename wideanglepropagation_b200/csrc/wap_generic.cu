@@ -457,47 +457,6 @@ __global__ void __launch_bounds__(kRowThreads) gen_wpm_row_kernel(const GenWpmRo
   }
 }
 
-// wpm_bins_kernel for any pixel count (no float4 loads)
-static __global__ void __launch_bounds__(1024) gen_wpm_bins_kernel(const WpmBinsArgs a) {
-  const int s = blockIdx.x, d = blockIdx.y;
-  const float* vs = a.V + ((long long)d * a.n_slices + s) * a.n_px;
-  float lo = 3.0e38f, hi = -3.0e38f;
-  for (int i = threadIdx.x; i < a.n_px; i += blockDim.x) {
-    const float dn = refr_minus_one(__ldg(vs + i), a.ri_a, a.ri_inv_den);
-    lo = fminf(lo, dn);
-    hi = fmaxf(hi, dn);
-  }
-  __shared__ float slo[32], shi[32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-  }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) {
-    slo[w] = lo;
-    shi[w] = hi;
-  }
-  __syncthreads();
-  if (w == 0) {
-    const int nw = blockDim.x >> 5;
-    lo = l < nw ? slo[l] : 3.0e38f;
-    hi = l < nw ? shi[l] : -3.0e38f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
-    float* out = a.refs + ((long long)d * a.n_slices + s) * a.K;
-    const double dlo = lo, dhi = hi;
-    for (int k = l; k < a.K; k += 32) {
-      const double tk = (k == a.K - 1) ? 1.0 : (double)k * (1.0 / (double)(a.K - 1));
-      const double tp = (a.power == 1.0) ? tk : pow(tk, a.power);
-      out[k] = (float)(dlo + (dhi - dlo) * tp);
-    }
-  }
-}
-
 // ----------------------------------------------------------------------------
 // launches: one instance per transform size m (E = 8 up to 128 points, else 16)
 // ----------------------------------------------------------------------------
@@ -730,16 +689,12 @@ int generic_fresnel_forward(wap_plan* p, const float* V, int n_slices, int n_dra
 
 int generic_wpm_forward(wap_plan* p, const float* V, int n_slices, int n_draws, const int32_t* draw,
                         const float* psi0, int n_probes, int psi0_per_probe, const int32_t* positions, double dz,
-                        double energy, double sampling_y, double sampling_x, double power_spacing, float* exit,
-                        float* dp, float* stack, cudaStream_t st) {
+                        double energy, const WpmNodeScalars& nodes, float* exit, float* dp, float* stack,
+                        cudaStream_t st) {
   const Physics ph = physics(energy, dz);
   const int K = p->n_bins;
   const long long plane = (long long)p->ny * p->nx;
   cudaError_t e;
-  WpmBinsArgs bargs{V, p->refs, (int)plane, n_slices, K, (float)ph.ri_a, (float)ph.ri_inv_den, power_spacing};
-  count_launch();
-  gen_wpm_bins_kernel<<<dim3(n_slices, n_draws), 1024, 0, st>>>(bargs);
-  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "generic wpm bins");
   GenRowArgs r{};
   r.psi = reinterpret_cast<float2*>(exit);
   r.psi_bstride = plane;

@@ -19,6 +19,8 @@ struct Detector {
   __host__ __device__ long long plane() const { return (long long)ny * nx; }
 };
 
+struct WpmSlice;   // a slice's WPM record (wap_wpm_nodes.cuh)
+
 // One axis of a grid that is not a power of two (wap_generic.cu): a length-n
 // DFT as Bluestein's chirp convolution through an m-point FFT (m the power of
 // two >= 2n - 1), or, for a power-of-two axis of such a grid, the plain
@@ -50,6 +52,10 @@ struct wap_plan {
   double hvac_key[4] = {0, 0, 0, 0};        // (dy, dx, dz, energy) of hvac
   float* refs = nullptr;                    // (draws, n_slices, n_bins)
   size_t refs_cap = 0;
+  wap::WpmSlice* slices = nullptr;          // (draws, n_slices) interpolation records
+  size_t slices_cap = 0;
+  float4* wn_tw_row = nullptr;              // (nx, 8) and (ny, 8) twiddles of the interpolating passes
+  float4* wn_tw_col = nullptr;
   float2* ttab = nullptr;                   // transmission table (draws, n_slices, ny, nx)
   size_t ttab_cap = 0;
   wap::Detector det;                        // diffraction-pattern window (wap_plan_set_detector)
@@ -113,6 +119,15 @@ int chain_forward(wap_plan* p, const RowArgs& r, const ColArgs& c, int n_probes,
 int cluster_forward(wap_plan* p, const RowArgs& r, const ColArgs& c, int n_probes, int n_slices, float2* stack,
                     cudaStream_t st);
 
+// reference values and interpolation records of every slice (wap_wpm.cu)
+struct WpmNodeScalars {
+  bool nodes = false;   // records may hold interpolation nodes (else every slice forms its K reference fields)
+  // the slope dz / (2 sqrt(qbar)) taken out per pixel, and qbar - k0^2, 1 / qbar, 1 / sqrt(qbar)
+  float kappa = 0.f, dq = 0.f, inv_qbar = 0.f, inv_root_qbar = 0.f;
+  float2 kk = {0.f, 0.f};   // kappa k0^2, hi and lo parts
+};
+int wpm_node_twiddles(wap_plan* p);
+
 // grids that are not powers of two (wap_generic.cu)
 bool generic_size_supported(int n);
 int generic_axis_create(GenAxis* ax, int n);
@@ -123,8 +138,8 @@ int generic_fresnel_forward(wap_plan* p, const float* V, int n_slices, int n_dra
                             float* stack, cudaStream_t st);
 int generic_wpm_forward(wap_plan* p, const float* V, int n_slices, int n_draws, const int32_t* draw,
                         const float* psi0, int n_probes, int psi0_per_probe, const int32_t* positions, double dz,
-                        double energy, double sampling_y, double sampling_x, double power_spacing, float* exit,
-                        float* dp, float* stack, cudaStream_t st);
+                        double energy, const WpmNodeScalars& nodes, float* exit, float* dp, float* stack,
+                        cudaStream_t st);
 ColArgs base_col_args(const wap_plan* p, const float* H, const float* H_lo);
 RowArgs base_row_args(const wap_plan* p, const Physics& ph, const float* V, int n_slices, const int32_t* draw);
 int build_trans_table(wap_plan* p, const float* V, int n_slices, int n_draws, const RowArgs& r, cudaStream_t st);

@@ -165,6 +165,26 @@ __device__ __forceinline__ void pdl_wait_then_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Row and column passes go out with programmatic dependent launch (the
+// kernels wait for their predecessor first thing): in a chain of short,
+// latency-bound passes the next pass is already resident when one finishes
+// (C1 0.26 -> 0.19 ms per call).  The reference-field WPM passes launch normally:
+// their large CTAs parked early cost more than the launch latency saved (C3 12.5 vs 13.1 ms).
+template <class K, class A>
+static cudaError_t launch_pdl(K kern, dim3 grid, int threads, size_t smem, cudaStream_t st, const A& args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args);
+}
+
 // ----------------------------------------------------------------------------
 // row pass
 // ----------------------------------------------------------------------------
@@ -523,7 +543,7 @@ __device__ __forceinline__ float2 cis_small(float ph) {
 // with H_k = exp(i dz sqrt(n_k^2 k0^2 - k_perp^2)) and blends, per pixel, the
 // two fields that bracket the pixel's n with smoothstep weights.  Here:
 //   * bins live in delta = n - 1 (n_refs - 1 = dmin + (dmax - dmin) t^p,
-//     the same points), computed for all slices up front (wpm_bins_kernel);
+//     the same points), computed for all slices up front (wpm_slices_kernel);
 //   * H_k = Hvac * exp(i dz a_k / (kz_k + kz_0)), a_k = k0^2 dk (2 + dk),
 //     with Hvac = exp(i dz sqrt(k0^2 - k_perp^2)) tabulated in float64 on the
 //     device and rounded once; the small residual phase is formed in float32
@@ -531,73 +551,8 @@ __device__ __forceinline__ float2 cis_small(float ph) {
 //     branch of the reference directly;
 //   * wpm_col_kernel writes the K column-transformed fields, wpm_row_kernel
 //     finishes each field's inverse row transform and accumulates the blend.
-
-struct WpmBinsArgs {
-  const float* V;            // (draws, n_slices, ny, nx)
-  float* refs;               // (draws, n_slices, K) delta reference values
-  int n_px, n_slices, K;
-  float ri_a, ri_inv_den;
-  double power;
-};
-
-// one CTA per (slice, draw): min/max of delta over the slice, then the K
-// reference values delta_min + (delta_max - delta_min) t_k^p in float64.
-// Each thread keeps eight 16-byte loads in flight per trip: with one, the
-// slice's reduction is a chain of 64 memory latencies at 512^2.
-static __global__ void __launch_bounds__(1024) wpm_bins_kernel(const WpmBinsArgs a) {
-  constexpr int kInFlight = 8;
-  const int s = blockIdx.x, d = blockIdx.y;
-  const float4* v4 = reinterpret_cast<const float4*>(a.V + ((long long)d * a.n_slices + s) * a.n_px);
-  const int n4 = a.n_px >> 2, step = blockDim.x;
-  float lo = 3.0e38f, hi = -3.0e38f;
-  auto fold = [&](const float4 q) {
-    const float d0 = refr_minus_one(q.x, a.ri_a, a.ri_inv_den);
-    const float d1 = refr_minus_one(q.y, a.ri_a, a.ri_inv_den);
-    const float d2 = refr_minus_one(q.z, a.ri_a, a.ri_inv_den);
-    const float d3 = refr_minus_one(q.w, a.ri_a, a.ri_inv_den);
-    lo = fminf(lo, fminf(fminf(d0, d1), fminf(d2, d3)));
-    hi = fmaxf(hi, fmaxf(fmaxf(d0, d1), fmaxf(d2, d3)));
-  };
-  int i = threadIdx.x;
-  for (; i + (kInFlight - 1) * step < n4; i += kInFlight * step) {
-    float4 q[kInFlight];
-#pragma unroll
-    for (int u = 0; u < kInFlight; ++u) q[u] = __ldg(v4 + i + u * step);
-#pragma unroll
-    for (int u = 0; u < kInFlight; ++u) fold(q[u]);
-  }
-  for (; i < n4; i += step) fold(__ldg(v4 + i));
-  __shared__ float slo[32], shi[32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-  }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) {
-    slo[w] = lo;
-    shi[w] = hi;
-  }
-  __syncthreads();
-  if (w == 0) {
-    const int nw = blockDim.x >> 5;
-    lo = l < nw ? slo[l] : 3.0e38f;
-    hi = l < nw ? shi[l] : -3.0e38f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
-    float* out = a.refs + ((long long)d * a.n_slices + s) * a.K;
-    const double dlo = lo, dhi = hi;
-    for (int k = l; k < a.K; k += 32) {
-      // numpy linspace(0, 1, K): k * (1/(K-1)), last point exactly 1
-      const double tk = (k == a.K - 1) ? 1.0 : (double)k * (1.0 / (double)(a.K - 1));
-      const double tp = (a.power == 1.0) ? tk : pow(tk, a.power);
-      out[k] = (float)(dlo + (dhi - dlo) * tp);
-    }
-  }
-}
+// They serve grids that reach the evanescent edge; other calls form a few
+// interpolation nodes instead of the K fields (wap_wpm_nodes.cuh).
 
 struct WpmColArgs {
   const float2* psi;         // (B, ny, nx) row-transformed wave

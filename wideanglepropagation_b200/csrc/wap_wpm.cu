@@ -1,13 +1,16 @@
 // WPM adaptive-binning forward (propagation.py:215-256, :358-387).
 //
 // Launch sequence for N slices, all in place on the caller's exit buffer:
-//   wpm_bins_kernel            reference deltas of every slice (one launch)
+//   wpm_slices_kernel          reference deltas and record of every slice (one launch)
 //   row pass  (load, FFT)      psi0 -> row spectrum
 //   for s in 0..N-1:
-//     wpm_col_kernel  s        column FFT, K x (propagate, column IFFT) -> fields
-//     wpm_row_kernel  s        K x row IFFT, smoothstep blend -> wave after slice s,
+//     wpm_node_col_kernel s    column FFT, per field (factor, column IFFT) -> fields
+//     wpm_node_row_kernel s    per field row IFFT, blend -> wave after slice s,
 //                              then its row FFT (input of slice s+1)
 //   wpm_col_kernel (dp mode)   |fftshift(fft2(exit))|^2
+// with the fields of a few interpolation nodes (wap_wpm_nodes.cuh), or, for grids
+// that reach the evanescent edge, wpm_col_kernel / wpm_row_kernel with the fields
+// of the K reference indices.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -15,6 +18,7 @@
 
 #include "wap_internal.h"
 #include "wap_passes.cuh"
+#include "wap_wpm_nodes.cuh"
 
 namespace wap {
 
@@ -51,6 +55,243 @@ __global__ void wpm_vacuum_kernel(const HvacArgs a) {
   if (iy == 0) a.kx2[ix] = (float)(kx * kx);
 }
 
+// ----------------------------------------------------------------------------
+// launches of the interpolating passes: eight elements per thread at every size
+// ----------------------------------------------------------------------------
+constexpr int kNodeE = 8;
+
+template <class K>
+static cudaError_t node_smem(K kern, size_t smem) {
+  return smem > 48 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                          : cudaSuccess;
+}
+
+// Whether a pass of `lines` lines of n points leaves the chip waiting on each
+// warp's chain of transforms, so that a line's fields go to several groups: up to
+// two one-group warps per scheduler.  Measured per call, K = 16, split / not: one
+// 512^2 probe x 200 slices 3.53 / 4.41 ms, four 256^2 probes x 100 1.55 / 2.07 ms;
+// two 512^2 probes x 60 2.01 / 1.67 ms, one 1024^2 probe x 40 3.62 / 3.02 ms.
+static bool node_split(int n, long long lines) { return lines * (n / kNodeE) <= 148LL * 256; }
+
+template <int N, int G>
+static cudaError_t launch_node_col_t(const WpmNodeColArgs& a, int nb, cudaStream_t st) {
+  constexpr int T = N / kNodeE;
+  // columns per CTA: eight (64-byte row segments) within the thread limit, four
+  // when eight would leave SMs without a CTA
+  int w = 8;
+  while (w > 1 && (w * T * G > node_col_threads(N, G) || w > a.c.nx)) w >>= 1;
+  if (w == 8 && (long long)(a.c.nx / w) * nb < 148 && 4 * T >= 32) w = 4;
+  const size_t smem = (size_t)N * w * G * sizeof(float2) + FFTPlan<N, kNodeE>::TW_SIZE * sizeof(float4);
+  cudaError_t e = node_smem(wpm_node_col_kernel<N, kNodeE, G>, smem);
+  if (e != cudaSuccess) return e;
+  count_launch();
+  return launch_pdl(wpm_node_col_kernel<N, kNodeE, G>, dim3(a.c.nx / w, nb), w * T * G, smem, st, a);
+}
+
+template <int N, int G>
+static cudaError_t launch_node_row_t(const WpmNodeRowArgs& a, int nb, cudaStream_t st) {
+  constexpr int T = N / kNodeE;
+  // rows per CTA: kRowThreads threads per group (or half that with several
+  // groups), fewer while SMs would be left without two CTAs; whole warps
+  int rows = std::max(1, (G > 1 ? kRowThreads / 2 : kRowThreads) / T);
+  while (rows > 1 && (rows > a.r.ny || ((long long)(a.r.ny / rows) * nb < 296 && rows * T * G > 128 && rows * T > 32)))
+    rows >>= 1;
+  // twiddles, pixel blends (28 bytes each), the groups' exchange segments, references
+  const size_t smem = FFTPlan<N, kNodeE>::TW_SIZE * sizeof(float4) + (size_t)rows * N * 28 +
+                      (size_t)rows * G * RowCfg<N, kNodeE>::PADN * sizeof(float2) + (size_t)a.r.K * sizeof(float);
+  cudaError_t e = node_smem(wpm_node_row_kernel<N, kNodeE, G>, smem);
+  if (e != cudaSuccess) return e;
+  count_launch();
+  return launch_pdl(wpm_node_row_kernel<N, kNodeE, G>, dim3(a.r.ny / rows, nb), rows * G * T, smem, st, a);
+}
+
+#define WAP_NODE_SIZES(M) M(32) M(64) M(128) M(256) M(512) M(1024) M(2048)
+#define WAP_NODE_COL(M)                                                                                   \
+  case M:                                                                                                 \
+    return node_split(M, (long long)a.c.nx * nb) ? launch_node_col_t<M, node_col_groups(M)>(a, nb, st)    \
+                                                 : launch_node_col_t<M, 1>(a, nb, st);
+#define WAP_NODE_ROW(M)                                                                                   \
+  case M:                                                                                                 \
+    return node_split(M, (long long)a.r.ny * nb) ? launch_node_row_t<M, node_row_groups(M)>(a, nb, st)    \
+                                                 : launch_node_row_t<M, 1>(a, nb, st);
+static cudaError_t launch_node_col(int n, const WpmNodeColArgs& a, int nb, cudaStream_t st) {
+  switch (n) { WAP_NODE_SIZES(WAP_NODE_COL) default: return cudaErrorInvalidValue; }
+}
+static cudaError_t launch_node_row(int n, const WpmNodeRowArgs& a, int nb, cudaStream_t st) {
+  switch (n) { WAP_NODE_SIZES(WAP_NODE_ROW) default: return cudaErrorInvalidValue; }
+}
+
+// twiddles of the interpolating passes (plan creation)
+int wpm_node_twiddles(wap_plan* p) {
+  for (int which = 0; which < 2; ++which) {
+    float4*& d = which == 0 ? p->wn_tw_row : p->wn_tw_col;
+    const std::vector<float4> h = twiddle_table(which == 0 ? p->nx : p->ny, kNodeE);
+    cudaError_t e = cudaMalloc(&d, h.size() * sizeof(float4));
+    if (e == cudaSuccess) e = cudaMemcpy(d, h.data(), h.size() * sizeof(float4), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+      cudaFree(d);
+      d = nullptr;
+      return cuda_fail(e, "WPM twiddles");
+    }
+  }
+  return WAP_OK;
+}
+
+// largest (2 pi f)^2 of numpy.fft.fftfreq(n, d)
+static double k2_max(int n, double d) {
+  const double k = 2.0 * M_PI * (double)(n / 2) / ((double)n * d);
+  return k * k;
+}
+
+// Reference values and records of every slice.  Interpolation needs a grid that
+// stays clear of the evanescent edge (k0^2 above the largest k_perp^2).  Its passes
+// also serve the slices that then find no node count below K, with their K
+// reference fields: few bins, where they beat the split reference kernels (512^2,
+// K = 4: 0.83 against 1.84 ms for 40 slices); the evanescent grids keep those,
+// which share many bins out over more CTAs (256^2, K = 128: 1.7 against 4.1 ms for 20).
+static int wpm_slices(wap_plan* p, const float* V, int n_slices, int n_draws, const Physics& ph, double dz,
+                      double sampling_y, double sampling_x, double power_spacing, WpmNodeScalars* out,
+                      cudaStream_t st) {
+  const int K = p->n_bins;
+  const size_t rows = (size_t)n_draws * n_slices;
+  cudaError_t e;
+  if (rows * K > p->refs_cap) {
+    cudaFree(p->refs);
+    p->refs = nullptr;
+    p->refs_cap = 0;
+    if ((e = cudaMalloc(&p->refs, rows * K * sizeof(float))) != cudaSuccess) return cuda_fail(e, "cudaMalloc(refs)");
+    p->refs_cap = rows * K;
+  }
+  if (rows > p->slices_cap) {
+    cudaFree(p->slices);
+    p->slices = nullptr;
+    p->slices_cap = 0;
+    if ((e = cudaMalloc(&p->slices, rows * sizeof(WpmSlice))) != cudaSuccess)
+      return cuda_fail(e, "cudaMalloc(WPM records)");
+    p->slices_cap = rows;
+  }
+  const double qmin = ph.k0 * ph.k0 - (k2_max(p->ny, sampling_y) + k2_max(p->nx, sampling_x));
+  out->nodes = qmin > 0.0 && std::fabs(dz) >= 1e-6;
+  if (out->nodes) {
+    const double inv_root = 0.5 * (1.0 / std::sqrt(qmin) + 1.0 / ph.k0), qbar = 1.0 / (inv_root * inv_root);
+    out->kappa = (float)(0.5 * dz * inv_root);
+    const double kk = 0.5 * dz * inv_root * ph.k0 * ph.k0;
+    out->kk = make_float2((float)kk, (float)(kk - (double)(float)kk));
+    out->dq = (float)(qbar - ph.k0 * ph.k0);
+    out->inv_qbar = (float)(1.0 / qbar);
+    out->inv_root_qbar = (float)inv_root;
+  }
+  const long long plane = (long long)p->ny * p->nx;
+  const WpmSlicesArgs a{V, p->refs, p->slices, (int)plane, n_slices, K, out->nodes ? 1 : 0, (float)ph.ri_a,
+                        (float)ph.ri_inv_den, power_spacing, ph.k0, qmin, dz};
+  const ProfToken tok = prof_begin(WAP_KIND_WPM_BINS, st);
+  count_launch();
+  wpm_slices_kernel<<<dim3(n_slices * kWpmCluster, n_draws), kWpmSliceThreads, 0, st>>>(a);
+  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "wpm_slices_kernel");
+  prof_end(tok, st, 4.0 * plane * n_slices * n_draws);
+  return WAP_OK;
+}
+
+// Slices [0, n_slices) of nb probes from the fields of interpolation nodes.
+static int node_slices(const wap_plan* p, const WpmNodeScalars& nodes, const WpmColArgs& c, const WpmRowArgs& w,
+                       double power, int n_slices, int nb, float2* stack, cudaStream_t st) {
+  const long long plane = (long long)p->ny * p->nx;
+  WpmNodeColArgs nc{c, p->slices, nodes.kappa, nodes.dq, nodes.inv_qbar, nodes.inv_root_qbar, 4.0f / (c.dz * c.dz)};
+  nc.c.tw = p->wn_tw_col;
+  WpmNodeRowArgs nr{w, p->slices, nodes.kk, power == 1.0 ? 1 : power == 2.0 ? 2 : 0};
+  nr.r.tw = p->wn_tw_row;
+  cudaError_t e;
+  for (int s = 0; s < n_slices; ++s) {
+    nc.c.slice = nr.r.slice = s;
+    ProfToken tok = prof_begin(WAP_KIND_WPM_COL, st);
+    if ((e = launch_node_col(p->ny, nc, nb, st)) != cudaSuccess) return cuda_fail(e, "wpm column pass");
+    // wave in, one field out at least, vacuum propagator once
+    prof_end(tok, st, 16.0 * plane * nb + 8.0 * plane);
+    nr.r.last = (s == n_slices - 1);
+    nr.r.snap = stack ? stack + (long long)s * plane : nullptr;
+    tok = prof_begin(WAP_KIND_WPM_ROW, st);
+    if ((e = launch_node_row(p->nx, nr, nb, st)) != cudaSuccess) return cuda_fail(e, "wpm row pass");
+    prof_end(tok, st, (20.0 + (nr.r.last ? 8.0 : 0.0) + (nr.r.snap ? 8.0 : 0.0)) * plane * nb);
+  }
+  return WAP_OK;
+}
+
+// The same from the fields of the K reference indices.
+static int reference_slices(const wap_plan* p, const Physics& ph, const float* V, const int32_t* draw, WpmColArgs c,
+                            WpmRowArgs w, int n_slices, int b0, int nb, float2* exit, float2* stack, cudaStream_t st) {
+  const int K = p->n_bins;
+  const long long plane = (long long)p->ny * p->nx;
+  const int rows = rows_per_cta(p->nx, p->row_e, p->ny);
+  cudaError_t e;
+  // Few probes leave most SMs idle (a 512^2 probe is 128 column and 128 row
+  // CTAs): then the K bins are split across CTA groups - each column CTA
+  // redoes the column FFT for its share of the bins, each row CTA blends the
+  // pixels whose left bin is in its share, and a row pass applies the row FFT.
+  // The group count minimises (waves of resident CTAs) x (transforms per CTA).
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+  const int col_slots = std::max(1, wpm_col_occupancy(p->ny, p->col_e, p->col_w, K)) * sms;
+  const int row_slots = std::max(1, wpm_row_occupancy(p->nx, p->row_e, rows, K)) * sms;
+  // Bins per group (the launched group count is ceil(units / per)).  Column
+  // CTA: 1 + per transforms; row CTA: K transforms unsplit, else per + 1 and
+  // the row pass that follows (counted as one more).
+  auto best_per = [&](long long ctas0, int slots, int units, bool col) {
+    int best = units;
+    double best_cost = 1e300;
+    for (int per = units; per >= 1; --per) {
+      const long long g = (units + per - 1) / per;
+      const double waves = std::ceil((double)(ctas0 * g) / slots);
+      const double work = col ? 1.0 + per : (g == 1 ? (double)K : per + 2.0);
+      if (waves * work < best_cost) {
+        best_cost = waves * work;
+        best = per;
+      }
+    }
+    return best;
+  };
+
+  c.kpg = best_per((long long)(p->nx / p->col_w) * nb, col_slots, K, true);
+  w.kpg = best_per((long long)(p->ny / rows) * nb, row_slots, K - 1, false);
+  const int gr = (K - 1 + w.kpg - 1) / w.kpg;
+  w.blend = gr > 1 ? p->blend : nullptr;
+  RowArgs fin = base_row_args(p, ph, V, n_slices, draw);   // the row FFT after a bin-split blend
+  fin.src = p->blend;
+  fin.src_bstride = plane;
+  fin.shifts = nullptr;
+  fin.flags = ROW_LOAD_SRC | ROW_FFT;
+  for (int s = 0; s < n_slices; ++s) {
+    c.slice = s;
+    c.dp_mode = 0;
+    ProfToken tok = prof_begin(WAP_KIND_WPM_COL, st);
+    if ((e = launch_wpm_col(p->ny, p->col_e, c, nb, p->col_w, st)) != cudaSuccess) return cuda_fail(e, "wpm column pass");
+    // wave in, K fields out, vacuum propagator once
+    prof_end(tok, st, (8.0 + 8.0 * K) * plane * nb + 8.0 * plane);
+    w.slice = s;
+    w.last = (s == n_slices - 1);
+    w.snap = stack ? stack + (long long)s * plane : nullptr;
+    tok = prof_begin(WAP_KIND_WPM_ROW, st);
+    if ((e = launch_wpm_row(p->nx, p->row_e, w, nb, rows, st)) != cudaSuccess) return cuda_fail(e, "wpm row pass");
+    // K fields in, potential, wave out (+ dp buffer on the last slice, + snapshot)
+    prof_end(tok, st, (8.0 * K + 4.0 + 8.0 + (w.last ? 8.0 : 0.0) + (w.snap ? 8.0 : 0.0)) * plane * nb);
+    if (w.blend) {
+      // row FFT of the blended wave; the spatial wave is this slice's snapshot
+      // (at the last slice: the exit wave, the transform going to the dp buffer)
+      fin.probe0 = b0;
+      fin.psi = w.last ? p->dpbuf : exit;
+      fin.psi_bstride = plane;
+      fin.snap = w.last ? exit : w.snap;
+      fin.snap_bstride = w.last ? plane : (long long)n_slices * plane;
+      if ((e = launch_row(p->nx, p->row_e, fin, nb, rows, st)) != cudaSuccess) return cuda_fail(e, "wpm row FFT");
+      if (w.last && w.snap &&
+          (e = cudaMemcpy2DAsync(w.snap + (long long)b0 * n_slices * plane, (size_t)n_slices * plane * sizeof(float2),
+                                 exit + (long long)b0 * plane, plane * sizeof(float2),
+                                 plane * sizeof(float2), nb, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
+        return cuda_fail(e, "wpm last snapshot");
+    }
+  }
+  return WAP_OK;
+}
+
 }  // namespace wap
 
 using namespace wap;
@@ -71,14 +312,6 @@ extern "C" int wap_wpm_fwd(wap_plan* p, const float* V, int n_slices, int n_draw
   const long long plane = (long long)p->ny * p->nx;
   cudaError_t e;
 
-  const size_t need = (size_t)n_draws * n_slices * K;
-  if (need > p->refs_cap) {
-    cudaFree(p->refs);
-    p->refs = nullptr;
-    p->refs_cap = 0;
-    if ((e = cudaMalloc(&p->refs, need * sizeof(float))) != cudaSuccess) return cuda_fail(e, "cudaMalloc(refs)");
-    p->refs_cap = need;
-  }
   const double key[4] = {sampling_y, sampling_x, dz, energy};
   if (!std::equal(key, key + 4, p->hvac_key)) {
     HvacArgs h{p->ny, p->nx, sampling_y, sampling_x, dz, ph.k0, p->hvac, p->hvac_lo, p->ky2, p->kx2};
@@ -87,18 +320,11 @@ extern "C" int wap_wpm_fwd(wap_plan* p, const float* V, int n_slices, int n_draw
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "wpm_vacuum_kernel");
     std::copy(key, key + 4, p->hvac_key);
   }
+  WpmNodeScalars nodes;
+  if ((rc = wpm_slices(p, V, n_slices, n_draws, ph, dz, sampling_y, sampling_x, power_spacing, &nodes, st))) return rc;
   if (p->generic)
     return generic_wpm_forward(p, V, n_slices, n_draws, draw, psi0, n_probes, psi0_per_probe, positions, dz, energy,
-                               sampling_y, sampling_x, power_spacing, exit, dp, stack, st);
-
-  WpmBinsArgs bargs{V, p->refs, (int)plane, n_slices, K, (float)ph.ri_a, (float)ph.ri_inv_den, power_spacing};
-  {
-    const ProfToken tok = prof_begin(WAP_KIND_WPM_BINS, st);
-    count_launch();
-    wpm_bins_kernel<<<dim3(n_slices, n_draws), 1024, 0, st>>>(bargs);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "wpm_bins_kernel");
-    prof_end(tok, st, 4.0 * plane * n_slices * n_draws);
-  }
+                               nodes, exit, dp, stack, st);
 
   // psi0 -> row spectrum
   RowArgs r = base_row_args(p, ph, V, n_slices, draw);
@@ -148,76 +374,14 @@ extern "C" int wap_wpm_fwd(wap_plan* p, const float* V, int n_slices, int n_draw
   w.snap_bstride = (long long)n_slices * plane;
   const int rows = rows_per_cta(p->nx, p->row_e, p->ny);
 
-  // Few probes leave most SMs idle (a 512^2 probe is 128 column and 128 row
-  // CTAs): then the K bins are split across CTA groups - each column CTA
-  // redoes the column FFT for its share of the bins, each row CTA blends the
-  // pixels whose left bin is in its share, and a row pass applies the row FFT.
-  // The group count minimises (waves of resident CTAs) x (transforms per CTA).
-  int sms = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
-  const int col_slots = std::max(1, wpm_col_occupancy(p->ny, p->col_e, p->col_w, K)) * sms;
-  const int row_slots = std::max(1, wpm_row_occupancy(p->nx, p->row_e, rows, K)) * sms;
-  // Bins per group (the launched group count is ceil(units / per)).  Column
-  // CTA: 1 + per transforms; row CTA: K transforms unsplit, else per + 1 and
-  // the row pass that follows (counted as one more).
-  auto best_per = [&](long long ctas0, int slots, int units, bool col) {
-    int best = units;
-    double best_cost = 1e300;
-    for (int per = units; per >= 1; --per) {
-      const long long g = (units + per - 1) / per;
-      const double waves = std::ceil((double)(ctas0 * g) / slots);
-      const double work = col ? 1.0 + per : (g == 1 ? (double)K : per + 2.0);
-      if (waves * work < best_cost) {
-        best_cost = waves * work;
-        best = per;
-      }
-    }
-    return best;
-  };
-
   for (int b0 = 0; b0 < n_probes; b0 += 65535) {
     const int nb = std::min(65535, n_probes - b0);
     c.probe0 = b0;
     w.probe0 = b0;
-    c.kpg = best_per((long long)(p->nx / p->col_w) * nb, col_slots, K, true);
-    w.kpg = best_per((long long)(p->ny / rows) * nb, row_slots, K - 1, false);
-    const int gr = (K - 1 + w.kpg - 1) / w.kpg;
-    w.blend = gr > 1 ? p->blend : nullptr;
-    RowArgs fin = base_row_args(p, ph, V, n_slices, draw);   // the row FFT after a bin-split blend
-    fin.src = p->blend;
-    fin.src_bstride = plane;
-    fin.shifts = nullptr;
-    fin.flags = ROW_LOAD_SRC | ROW_FFT;
-    for (int s = 0; s < n_slices; ++s) {
-      c.slice = s;
-      c.dp_mode = 0;
-      ProfToken tok = prof_begin(WAP_KIND_WPM_COL, st);
-      if ((e = launch_wpm_col(p->ny, p->col_e, c, nb, p->col_w, st)) != cudaSuccess) return cuda_fail(e, "wpm column pass");
-      // wave in, K fields out, vacuum propagator once
-      prof_end(tok, st, (8.0 + 8.0 * K) * plane * nb + 8.0 * plane);
-      w.slice = s;
-      w.last = (s == n_slices - 1);
-      w.snap = stack ? reinterpret_cast<float2*>(stack) + (long long)s * plane : nullptr;
-      tok = prof_begin(WAP_KIND_WPM_ROW, st);
-      if ((e = launch_wpm_row(p->nx, p->row_e, w, nb, rows, st)) != cudaSuccess) return cuda_fail(e, "wpm row pass");
-      // K fields in, potential, wave out (+ dp buffer on the last slice, + snapshot)
-      prof_end(tok, st, (8.0 * K + 4.0 + 8.0 + (w.last ? 8.0 : 0.0) + (w.snap ? 8.0 : 0.0)) * plane * nb);
-      if (w.blend) {
-        // row FFT of the blended wave; the spatial wave is this slice's snapshot
-        // (at the last slice: the exit wave, the transform going to the dp buffer)
-        fin.probe0 = b0;
-        fin.psi = w.last ? p->dpbuf : reinterpret_cast<float2*>(exit);
-        fin.psi_bstride = plane;
-        fin.snap = w.last ? reinterpret_cast<float2*>(exit) : w.snap;
-        fin.snap_bstride = w.last ? plane : (long long)n_slices * plane;
-        if ((e = launch_row(p->nx, p->row_e, fin, nb, rows, st)) != cudaSuccess) return cuda_fail(e, "wpm row FFT");
-        if (w.last && w.snap &&
-            (e = cudaMemcpy2DAsync(w.snap + (long long)b0 * n_slices * plane, (size_t)n_slices * plane * sizeof(float2),
-                                   reinterpret_cast<float2*>(exit) + (long long)b0 * plane, plane * sizeof(float2),
-                                   plane * sizeof(float2), nb, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
-          return cuda_fail(e, "wpm last snapshot");
-      }
-    }
+    rc = nodes.nodes ? node_slices(p, nodes, c, w, power_spacing, n_slices, nb, reinterpret_cast<float2*>(stack), st)
+                     : reference_slices(p, ph, V, draw, c, w, n_slices, b0, nb, reinterpret_cast<float2*>(exit),
+                                        reinterpret_cast<float2*>(stack), st);
+    if (rc) return rc;
     if (dp) {
       WpmColArgs d = c;
       d.psi = p->dpbuf;
