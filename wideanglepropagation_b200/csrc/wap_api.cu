@@ -374,8 +374,8 @@ int wap_plan_create(wap_plan** out, int ny, int nx, int max_batch, int op, int n
   p->col_e = ny >= 64 ? 16 : 8;
   p->col_w = default_col_w(ny, p->col_e, nx);
   p->generic = generic;
-  int rc = generic ? generic_axis_create(&p->gen_x, nx) : upload_twiddles(p);
-  if (rc == WAP_OK && generic) rc = generic_axis_create(&p->gen_y, ny);
+  int rc = generic ? generic_axis_create(&p->gen_x, nx, op == WAP_OP_WPM) : upload_twiddles(p);
+  if (rc == WAP_OK && generic) rc = generic_axis_create(&p->gen_y, ny, op == WAP_OP_WPM);
   if (rc != WAP_OK) {
     plan_free(p);   // keeps the failure's message
     return rc;
@@ -586,9 +586,14 @@ int build_trans_table(wap_plan* p, const float* V, int n_slices, int n_draws, co
   const long long n4 = (long long)need / 4;
   const ProfToken tok = prof_begin(WAP_KIND_TRANS, st);
   count_launch();
-  trans_table_kernel<<<(unsigned)std::min<long long>((n4 + 255) / 256, 148LL * 16), 256, 0, st>>>(
-      V, p->ttab, n4, r.ri_a, r.ri_inv_den, r.kphase);
-  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "trans_table_kernel");
+  if (p->generic) {   // any pixel count: no 16-byte loads
+    e = gen_trans_table(V, p->ttab, (long long)need, r, st);
+  } else {
+    trans_table_kernel<<<(unsigned)std::min<long long>((n4 + 255) / 256, 148LL * 16), 256, 0, st>>>(
+        V, p->ttab, n4, r.ri_a, r.ri_inv_den, r.kphase);
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) return cuda_fail(e, "trans_table_kernel");
   prof_end(tok, st, 12.0 * (double)need);
   return WAP_OK;
 }
@@ -605,13 +610,9 @@ int fresnel_forward(wap_plan* p, const float* V, int n_slices, int n_draws, cons
   if (rc) return rc;
   if (!H) return fail(WAP_ERR_ARG, "H must be a non-NULL device pointer");
   if (p->op != WAP_OP_FRESNEL_AS) return fail(WAP_ERR_ARG, "plan was not created for the Fresnel/AS path");
-  if (p->generic) {
-    if (ckpt)
-      return fail(WAP_ERR_UNSUPPORTED, "checkpointed forwards (gradients) need power-of-two grids, got %d x %d", p->ny,
-                  p->nx);
-    return generic_fresnel_forward(p, V, n_slices, n_draws, draw, psi0, n_probes, psi0_per_probe, positions, H, H_lo,
-                                   dz, energy, exit, dp, stack, st);
-  }
+  if (p->generic && ckpt)
+    return fail(WAP_ERR_UNSUPPORTED, "checkpointed forwards (gradients) need power-of-two grids, got %d x %d", p->ny,
+                p->nx);
   const Physics ph = physics(energy, dz);
   const long long plane = (long long)p->ny * p->nx;
   const int nck = ckpt ? (n_slices + ckpt_every - 1) / ckpt_every : 0;
@@ -639,6 +640,8 @@ int fresnel_forward(wap_plan* p, const float* V, int n_slices, int n_draws, cons
   } else {
     clear_error();
   }
+  if (p->generic)
+    return generic_fresnel_forward(p, r, c, n_slices, n_probes, reinterpret_cast<float2*>(stack), st);
   // few probes: every slice in one launch when the grid qualifies - the wave
   // held in a thread-block cluster (wap_cluster.cu), else a cooperative grid
   // (wap_chain.cu) - else one launch per pass below

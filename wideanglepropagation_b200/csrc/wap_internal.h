@@ -21,17 +21,20 @@ struct Detector {
 
 struct WpmSlice;   // a slice's WPM record (wap_wpm_nodes.cuh)
 
-// One axis of a grid that is not a power of two (wap_generic.cu): a length-n
-// DFT as Bluestein's chirp convolution through an m-point FFT (m the power of
-// two >= 2n - 1), or, for a power-of-two axis of such a grid, the plain
-// n-point FFT (m = n, blue = 0).  Device pointers; tables of float64 values
+// One axis of a grid that is not a power of two (wap_mixed.cuh): a length-n DFT
+// by stages of radices 2 .. 8, or as Bluestein's chirp convolution through such
+// transforms of a length m >= 2n - 1.  Device pointers; tables of float64 values
 // stored as float hi + lo parts.
 struct GenAxis {
-  int n = 0, m = 0, e = 16, blue = 0;
-  const float4* tw = nullptr;       // twiddles of the m-point FFT
+  int n = 0, m = 0, blue = 0, stages = 0;
+  int pow2 = 0;                     // Bluestein on the power-of-two core: tw holds the tables of 8 and
+                                    // (from tw_rev) 16 elements per thread; no stages
+  int radix[5] = {0, 0, 0, 0, 0};
+  int threads = 0;                  // per line: m / smallest radix, at most 256
+  int tw_rev = 0, tw_len = 0;       // offset of the reversed order's twiddles, entries of both
+  const float4* tw = nullptr;       // stage twiddles, radices in order, then in reverse order
   const float4* chirp = nullptr;    // (n) w_p = exp(-i pi p^2 / n)
-  const float4* bhat_f = nullptr;   // (m) fft_m(b) / m, b_q = conj(w_q) on the circular index range
-  const float4* bhat_i = nullptr;   // (m) fft_m(conj(b)) / m
+  const float4* bhat = nullptr;     // (m) fft_m(b) / m, b_q = conj(w_q) on the circular index range
 };
 }  // namespace wap
 
@@ -130,16 +133,18 @@ int wpm_node_twiddles(wap_plan* p);
 
 // grids that are not powers of two (wap_generic.cu)
 bool generic_size_supported(int n);
-int generic_axis_create(GenAxis* ax, int n);
+int generic_axis_create(GenAxis* ax, int n, bool wpm);
 void generic_axis_free(GenAxis* ax);
-int generic_fresnel_forward(wap_plan* p, const float* V, int n_slices, int n_draws, const int32_t* draw,
-                            const float* psi0, int n_probes, int psi0_per_probe, const int32_t* positions,
-                            const float* H, const float* H_lo, double dz, double energy, float* exit, float* dp,
-                            float* stack, cudaStream_t st);
-int generic_wpm_forward(wap_plan* p, const float* V, int n_slices, int n_draws, const int32_t* draw,
-                        const float* psi0, int n_probes, int psi0_per_probe, const int32_t* positions, double dz,
-                        double energy, const WpmNodeScalars& nodes, float* exit, float* dp, float* stack,
-                        cudaStream_t st);
+int generic_fresnel_forward(wap_plan* p, const RowArgs& r, const ColArgs& c, int n_slices, int n_probes,
+                            float2* stack, cudaStream_t st);
+cudaError_t gen_trans_table(const float* V, float2* ttab, long long n, const RowArgs& r, cudaStream_t st);
+int generic_wpm_forward(const wap_plan* p, const WpmColArgs& c, const WpmRowArgs& w, const WpmNodeScalars& nodes,
+                        double power, const float2* psi0, long long psi0_stride, const int32_t* positions,
+                        int n_slices, int n_probes, float* dp, float2* stack, cudaStream_t st);
+struct WpmNodeColArgs;
+struct WpmNodeRowArgs;
+WpmNodeColArgs wpm_node_col_args(const wap_plan* p, const WpmColArgs& c, const WpmNodeScalars& nodes);
+WpmNodeRowArgs wpm_node_row_args(const wap_plan* p, const WpmRowArgs& w, const WpmNodeScalars& nodes, double power);
 ColArgs base_col_args(const wap_plan* p, const float* H, const float* H_lo);
 RowArgs base_row_args(const wap_plan* p, const Physics& ph, const float* V, int n_slices, const int32_t* draw);
 int build_trans_table(wap_plan* p, const float* V, int n_slices, int n_draws, const RowArgs& r, cudaStream_t st);

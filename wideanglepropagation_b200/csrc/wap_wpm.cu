@@ -11,6 +11,7 @@
 // with the fields of a few interpolation nodes (wap_wpm_nodes.cuh), or, for grids
 // that reach the evanescent edge, wpm_col_kernel / wpm_row_kernel with the fields
 // of the K reference indices.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -53,6 +54,193 @@ __global__ void wpm_vacuum_kernel(const HvacArgs a) {
   a.hvac_lo[idx] = make_float2((float)(re - (double)rh), (float)(im - (double)ih));
   if (ix == 0) a.ky2[iy] = (float)(ky * ky);
   if (iy == 0) a.kx2[ix] = (float)(kx * kx);
+}
+
+// ----------------------------------------------------------------------------
+// the slices' reference values and records
+// ----------------------------------------------------------------------------
+struct WpmSlicesArgs {
+  const float* V;            // (draws, n_slices, ny, nx)
+  float* refs;               // (draws, n_slices, K) delta reference values
+  WpmSlice* rec;             // (draws, n_slices)
+  int n_px, n_slices, K;
+  int use_nodes;             // 0: no node records (grids that reach the evanescent edge, few bins)
+  float ri_a, ri_inv_den;
+  double power, k0, qmin, dz;
+};
+
+// Nodes needed for a range of half width ah whose largest |a| is amax, or 0 if
+// none up to `most` meets the tolerance.  Interpolation at r Chebyshev nodes of
+// [-1, 1] is off by at most max|f^(r)| / (2^(r-1) r!), f = exp(i g):
+// |f^(r)| / r! <= [z^r] exp(T z + sum_{m>=2} b_m z^m), T bounding the slope of
+// g (the variation of dz / (2 sqrt(q + a)) about kappa) and b_m the Taylor
+// coefficients of the square root, 2 theta |binom(1/2, m)| y^(m-1) with
+// theta = dz ah / (2 sqrt(q)) and y = ah / q at the smallest q.
+__device__ inline int wpm_node_count(double ah, double amax, double qmin, double k0, double dz, int most) {
+  const double qe = qmin - amax - ah;
+  const double y = ah / qe, th = fabs(dz) * ah / (2.0 * sqrt(qe));
+  double g[kWpmMaxNodes + 1], e[kWpmMaxNodes + 1];
+  g[1] = fabs(dz) * ah * (1.0 / sqrt(qmin) - 1.0 / k0) / 4.0 + th * amax / (2.0 * qe);
+  double b = 0.5, ym = 1.0;
+  for (int m = 2; m <= kWpmMaxNodes; ++m) {
+    b *= fabs(0.5 - (m - 1)) / m;
+    ym *= y;
+    g[m] = 2.0 * th * b * ym;
+  }
+  e[0] = 1.0;
+  double half = 2.0;
+  for (int r = 1; r <= kWpmMaxNodes; ++r) {
+    double s = 0.0;
+    for (int m = 1; m <= r; ++m) s += m * g[m] * e[r - m];
+    e[r] = s / r;
+    half *= 0.5;   // 2^-(r-1)
+    if (e[r] * half <= kWpmNodeTol) return r <= most ? r : 0;
+  }
+  return 0;
+}
+
+// Per (slice, draw): min / max over the slice of n^2 - 1 = V (a + V) inv_den, in
+// which delta = n - 1 grows (values without a real n are left out, as a NaN
+// delta always was), the K reference values delta_min + (delta_max - delta_min) t_k^p in
+// float64, and the slice's record.  One cluster of kWpmCluster CTAs per slice: each
+// reduces its share with eight 16-byte loads in flight per thread, the first CTA
+// folds the shares through distributed shared memory.  One CTA per slice (the
+// loads of a whole slice in one SM) took 41 us at 512^2 for any slice count.
+constexpr int kWpmCluster = 8;
+constexpr int kWpmSliceThreads = 512;
+
+static __global__ void __cluster_dims__(kWpmCluster, 1, 1) __launch_bounds__(kWpmSliceThreads)
+wpm_slices_kernel(const WpmSlicesArgs a) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  constexpr int kInFlight = 8;
+  const int s = blockIdx.x / kWpmCluster, d = blockIdx.y;
+  const long long row = (long long)d * a.n_slices + s;
+  const float* v = a.V + row * a.n_px;
+  float lo = INFINITY, hi = -INFINITY;
+  auto fold = [&](float volts) {
+    const float r = volts * (a.ri_a + volts) * a.ri_inv_den;
+    if (r >= -1.0f && r < INFINITY) {
+      lo = fminf(lo, r);
+      hi = fmaxf(hi, r);
+    }
+  };
+  const int first = (int)cl.block_rank() * kWpmSliceThreads + threadIdx.x, step = kWpmCluster * kWpmSliceThreads;
+  if ((a.n_px & 3) == 0 && (reinterpret_cast<uintptr_t>(a.V) & 15) == 0) {
+    const float4* v4 = reinterpret_cast<const float4*>(v);
+    const int n4 = a.n_px >> 2;
+    int i = first;
+    for (; i + (kInFlight - 1) * step < n4; i += kInFlight * step) {
+      float4 q[kInFlight];
+#pragma unroll
+      for (int u = 0; u < kInFlight; ++u) q[u] = __ldg(v4 + i + u * step);
+#pragma unroll
+      for (int u = 0; u < kInFlight; ++u) { fold(q[u].x); fold(q[u].y); fold(q[u].z); fold(q[u].w); }
+    }
+    for (; i < n4; i += step) {
+      const float4 q = __ldg(v4 + i);
+      fold(q.x); fold(q.y); fold(q.z); fold(q.w);
+    }
+  } else {
+    for (int i = first; i < a.n_px; i += step) fold(__ldg(v + i));
+  }
+  __shared__ float slo[32], shi[32];
+  __shared__ float part[2];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l == 0) {
+    slo[w] = lo;
+    shi[w] = hi;
+  }
+  __syncthreads();
+  if (w == 0) {
+    constexpr int nw = kWpmSliceThreads / 32;
+    lo = l < nw ? slo[l] : INFINITY;
+    hi = l < nw ? shi[l] : -INFINITY;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (l == 0) {
+      part[0] = lo;
+      part[1] = hi;
+    }
+  }
+  cl.sync();
+  if (cl.block_rank() == 0 && w < 2) {
+    lo = INFINITY;
+    hi = -INFINITY;
+    if (l < kWpmCluster) {
+      const float* p = cl.map_shared_rank(part, l);
+      lo = p[0];
+      hi = p[1];
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    lo = __shfl_sync(0xffffffffu, lo, 0);
+    hi = __shfl_sync(0xffffffffu, hi, 0);
+    const double dlo = wpm_delta(lo), dhi = wpm_delta(hi);
+    if (w == 0) {
+      float* out = a.refs + row * a.K;
+      for (int k = l; k < a.K; k += 32) {
+        // numpy linspace(0, 1, K): k * (1/(K-1)), last point exactly 1
+        const double tk = (k == a.K - 1) ? 1.0 : (double)k * (1.0 / (double)(a.K - 1));
+        const double tp = (a.power == 1.0) ? tk : pow(tk, a.power);
+        out[k] = (float)(dlo + (dhi - dlo) * tp);
+      }
+    } else if (l == 0) {
+      int nf = a.K, nodes = 0;
+      float fxc = 0.f, finv = 0.f, fa0 = 0.f;
+      const double k02 = a.k0 * a.k0;
+      const double alo = k02 * dlo * (2.0 + dlo), ahi = k02 * dhi * (2.0 + dhi);
+      const double ac = 0.5 * (alo + ahi), ah = 0.5 * (ahi - alo), amax = fmax(fabs(alo), fabs(ahi));
+      // (a comparison with a NaN is false: such slices keep the K references)
+      if (a.use_nodes && ah >= 0.0 && amax <= a.qmin * 0.125 && dlo > -0.5) {
+        const int n = wpm_node_count(ah, amax, a.qmin, a.k0, a.dz, min(kWpmMaxNodes, a.K - 1));
+        if (n > 0) {
+          nf = n;
+          nodes = 1;
+          fxc = (float)(ac / k02);
+          finv = ah > 0.0 ? (float)(k02 / ah) : 0.f;
+          const int c = n >> 1;   // the node nearest the centre
+          double tau[kWpmMaxNodes];
+          for (int j = 0; j < n; ++j) {
+            const int m = j == 0 ? c : (j <= c ? j - 1 : j);
+            tau[j] = (2 * m + 1 == n) ? 0.0 : cos((2 * m + 1) * M_PI / (2.0 * n));
+          }
+          fa0 = (float)(ac + ah * tau[0]);
+          for (int j = 0; j < n; ++j) {
+            double p = 1.0;
+            int i = 0;
+            for (int m = 0; m < n; ++m) {
+              if (m == j) continue;
+              p *= tau[j] - tau[m];
+              a.rec[row].other[j][i++] = (float)tau[m];
+            }
+            a.rec[row].da[j] = (float)(ah * (tau[j] - tau[0]));
+            a.rec[row].bw[j] = (float)(1.0 / p);
+          }
+        }
+      }
+      WpmSlice& r = a.rec[row];
+      r.nf = nf;
+      r.nodes = nodes;
+      r.xc = fxc;
+      r.inv_xh = finv;
+      r.a0 = fa0;
+      r.dlo = (float)dlo;
+      r.inv_range = dhi > dlo ? (float)(1.0 / (dhi - dlo)) : 0.f;
+    }
+  }
+  cl.sync();   // the shares stay readable until the first CTA has them
 }
 
 // ----------------------------------------------------------------------------
@@ -192,14 +380,24 @@ static int wpm_slices(wap_plan* p, const float* V, int n_slices, int n_draws, co
   return WAP_OK;
 }
 
+WpmNodeColArgs wpm_node_col_args(const wap_plan* p, const WpmColArgs& c, const WpmNodeScalars& nodes) {
+  WpmNodeColArgs n{c,          p->slices,      nodes.kappa,         nodes.dq, nodes.inv_qbar, nodes.inv_root_qbar,
+                   4.0f / (c.dz * c.dz)};
+  n.c.tw = p->wn_tw_col;
+  return n;
+}
+WpmNodeRowArgs wpm_node_row_args(const wap_plan* p, const WpmRowArgs& w, const WpmNodeScalars& nodes, double power) {
+  WpmNodeRowArgs n{w, p->slices, nodes.kk, power == 1.0 ? 1 : power == 2.0 ? 2 : 0};
+  n.r.tw = p->wn_tw_row;
+  return n;
+}
+
 // Slices [0, n_slices) of nb probes from the fields of interpolation nodes.
 static int node_slices(const wap_plan* p, const WpmNodeScalars& nodes, const WpmColArgs& c, const WpmRowArgs& w,
                        double power, int n_slices, int nb, float2* stack, cudaStream_t st) {
   const long long plane = (long long)p->ny * p->nx;
-  WpmNodeColArgs nc{c, p->slices, nodes.kappa, nodes.dq, nodes.inv_qbar, nodes.inv_root_qbar, 4.0f / (c.dz * c.dz)};
-  nc.c.tw = p->wn_tw_col;
-  WpmNodeRowArgs nr{w, p->slices, nodes.kk, power == 1.0 ? 1 : power == 2.0 ? 2 : 0};
-  nr.r.tw = p->wn_tw_row;
+  WpmNodeColArgs nc = wpm_node_col_args(p, c, nodes);
+  WpmNodeRowArgs nr = wpm_node_row_args(p, w, nodes, power);
   cudaError_t e;
   for (int s = 0; s < n_slices; ++s) {
     nc.c.slice = nr.r.slice = s;
@@ -322,10 +520,6 @@ extern "C" int wap_wpm_fwd(wap_plan* p, const float* V, int n_slices, int n_draw
   }
   WpmNodeScalars nodes;
   if ((rc = wpm_slices(p, V, n_slices, n_draws, ph, dz, sampling_y, sampling_x, power_spacing, &nodes, st))) return rc;
-  if (p->generic)
-    return generic_wpm_forward(p, V, n_slices, n_draws, draw, psi0, n_probes, psi0_per_probe, positions, dz, energy,
-                               nodes, exit, dp, stack, st);
-
   // psi0 -> row spectrum
   RowArgs r = base_row_args(p, ph, V, n_slices, draw);
   r.psi = reinterpret_cast<float2*>(exit);
@@ -334,7 +528,7 @@ extern "C" int wap_wpm_fwd(wap_plan* p, const float* V, int n_slices, int n_draw
   r.src_bstride = psi0_per_probe ? plane : 0;
   r.shifts = positions;
   r.flags = ROW_LOAD_SRC | ROW_FFT;
-  if ((e = row_chunks(p, r, n_probes, st)) != cudaSuccess) return cuda_fail(e, "row pass");
+  if (!p->generic && (e = row_chunks(p, r, n_probes, st)) != cudaSuccess) return cuda_fail(e, "row pass");
 
   WpmColArgs c{};
   c.psi = reinterpret_cast<const float2*>(exit);
@@ -374,6 +568,9 @@ extern "C" int wap_wpm_fwd(wap_plan* p, const float* V, int n_slices, int n_draw
   w.snap_bstride = (long long)n_slices * plane;
   const int rows = rows_per_cta(p->nx, p->row_e, p->ny);
 
+  if (p->generic)
+    return generic_wpm_forward(p, c, w, nodes, power_spacing, r.src, r.src_bstride, positions, n_slices, n_probes, dp,
+                               reinterpret_cast<float2*>(stack), st);
   for (int b0 = 0; b0 < n_probes; b0 += 65535) {
     const int nb = std::min(65535, n_probes - b0);
     c.probe0 = b0;

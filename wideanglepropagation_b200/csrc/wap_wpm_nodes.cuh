@@ -23,8 +23,6 @@
 // (|.| ~ 1e-3 |G_c|): sum_j l_j = 1, so u = exp(i kappa a) (G_c + sum l_j (G_j - G_c)),
 // and the rounding of the r - 1 further transforms is scaled down with them.
 #pragma once
-#include <cooperative_groups.h>
-
 #include "wap_passes.cuh"
 
 namespace wap {
@@ -49,196 +47,12 @@ struct WpmSlice {
   float other[kWpmMaxNodes][kWpmMaxNodes];   // [j]: the nf - 1 node positions tau_m, m != j
 };
 
-struct WpmSlicesArgs {
-  const float* V;            // (draws, n_slices, ny, nx)
-  float* refs;               // (draws, n_slices, K) delta reference values
-  WpmSlice* rec;             // (draws, n_slices)
-  int n_px, n_slices, K;
-  int use_nodes;             // 0: no node records (grids that reach the evanescent edge, few bins)
-  float ri_a, ri_inv_den;
-  double power, k0, qmin, dz;
-};
-
 // delta = sqrt(1 + r) - 1 of r = n^2 - 1: the series of the square root for
 // |r| <= 1/64 (truncation 4e-11 of delta), where all but absurd potentials lie
 __device__ __forceinline__ float wpm_delta(float r) {
   if (fabsf(r) <= 0.015625f)
     return r * fmaf(r, fmaf(r, fmaf(r, fmaf(r, 0.02734375f, -0.0390625f), 0.0625f), -0.125f), 0.5f);
   return r / (sqrtf(1.0f + r) + 1.0f);
-}
-
-// Nodes needed for a range of half width ah whose largest |a| is amax, or 0 if
-// none up to `most` meets the tolerance.  Interpolation at r Chebyshev nodes of
-// [-1, 1] is off by at most max|f^(r)| / (2^(r-1) r!), f = exp(i g):
-// |f^(r)| / r! <= [z^r] exp(T z + sum_{m>=2} b_m z^m), T bounding the slope of
-// g (the variation of dz / (2 sqrt(q + a)) about kappa) and b_m the Taylor
-// coefficients of the square root, 2 theta |binom(1/2, m)| y^(m-1) with
-// theta = dz ah / (2 sqrt(q)) and y = ah / q at the smallest q.
-__device__ inline int wpm_node_count(double ah, double amax, double qmin, double k0, double dz, int most) {
-  const double qe = qmin - amax - ah;
-  const double y = ah / qe, th = fabs(dz) * ah / (2.0 * sqrt(qe));
-  double g[kWpmMaxNodes + 1], e[kWpmMaxNodes + 1];
-  g[1] = fabs(dz) * ah * (1.0 / sqrt(qmin) - 1.0 / k0) / 4.0 + th * amax / (2.0 * qe);
-  double b = 0.5, ym = 1.0;
-  for (int m = 2; m <= kWpmMaxNodes; ++m) {
-    b *= fabs(0.5 - (m - 1)) / m;
-    ym *= y;
-    g[m] = 2.0 * th * b * ym;
-  }
-  e[0] = 1.0;
-  double half = 2.0;
-  for (int r = 1; r <= kWpmMaxNodes; ++r) {
-    double s = 0.0;
-    for (int m = 1; m <= r; ++m) s += m * g[m] * e[r - m];
-    e[r] = s / r;
-    half *= 0.5;   // 2^-(r-1)
-    if (e[r] * half <= kWpmNodeTol) return r <= most ? r : 0;
-  }
-  return 0;
-}
-
-// Per (slice, draw): min / max over the slice of n^2 - 1 = V (a + V) inv_den, in
-// which delta = n - 1 grows (values without a real n are left out, as a NaN
-// delta always was), the K reference values delta_min + (delta_max - delta_min) t_k^p in
-// float64, and the slice's record.  One cluster of kWpmCluster CTAs per slice: each
-// reduces its share with eight 16-byte loads in flight per thread, the first CTA
-// folds the shares through distributed shared memory.  One CTA per slice (the
-// loads of a whole slice in one SM) took 41 us at 512^2 for any slice count.
-constexpr int kWpmCluster = 8;
-constexpr int kWpmSliceThreads = 512;
-
-static __global__ void __cluster_dims__(kWpmCluster, 1, 1) __launch_bounds__(kWpmSliceThreads)
-wpm_slices_kernel(const WpmSlicesArgs a) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cl = cg::this_cluster();
-  constexpr int kInFlight = 8;
-  const int s = blockIdx.x / kWpmCluster, d = blockIdx.y;
-  const long long row = (long long)d * a.n_slices + s;
-  const float* v = a.V + row * a.n_px;
-  float lo = INFINITY, hi = -INFINITY;
-  auto fold = [&](float volts) {
-    const float r = volts * (a.ri_a + volts) * a.ri_inv_den;
-    if (r >= -1.0f && r < INFINITY) {
-      lo = fminf(lo, r);
-      hi = fmaxf(hi, r);
-    }
-  };
-  const int first = (int)cl.block_rank() * kWpmSliceThreads + threadIdx.x, step = kWpmCluster * kWpmSliceThreads;
-  if ((a.n_px & 3) == 0 && (reinterpret_cast<uintptr_t>(a.V) & 15) == 0) {
-    const float4* v4 = reinterpret_cast<const float4*>(v);
-    const int n4 = a.n_px >> 2;
-    int i = first;
-    for (; i + (kInFlight - 1) * step < n4; i += kInFlight * step) {
-      float4 q[kInFlight];
-#pragma unroll
-      for (int u = 0; u < kInFlight; ++u) q[u] = __ldg(v4 + i + u * step);
-#pragma unroll
-      for (int u = 0; u < kInFlight; ++u) { fold(q[u].x); fold(q[u].y); fold(q[u].z); fold(q[u].w); }
-    }
-    for (; i < n4; i += step) {
-      const float4 q = __ldg(v4 + i);
-      fold(q.x); fold(q.y); fold(q.z); fold(q.w);
-    }
-  } else {
-    for (int i = first; i < a.n_px; i += step) fold(__ldg(v + i));
-  }
-  __shared__ float slo[32], shi[32];
-  __shared__ float part[2];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-  }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) {
-    slo[w] = lo;
-    shi[w] = hi;
-  }
-  __syncthreads();
-  if (w == 0) {
-    constexpr int nw = kWpmSliceThreads / 32;
-    lo = l < nw ? slo[l] : INFINITY;
-    hi = l < nw ? shi[l] : -INFINITY;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
-    if (l == 0) {
-      part[0] = lo;
-      part[1] = hi;
-    }
-  }
-  cl.sync();
-  if (cl.block_rank() == 0 && w < 2) {
-    lo = INFINITY;
-    hi = -INFINITY;
-    if (l < kWpmCluster) {
-      const float* p = cl.map_shared_rank(part, l);
-      lo = p[0];
-      hi = p[1];
-    }
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
-      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
-    lo = __shfl_sync(0xffffffffu, lo, 0);
-    hi = __shfl_sync(0xffffffffu, hi, 0);
-    const double dlo = wpm_delta(lo), dhi = wpm_delta(hi);
-    if (w == 0) {
-      float* out = a.refs + row * a.K;
-      for (int k = l; k < a.K; k += 32) {
-        // numpy linspace(0, 1, K): k * (1/(K-1)), last point exactly 1
-        const double tk = (k == a.K - 1) ? 1.0 : (double)k * (1.0 / (double)(a.K - 1));
-        const double tp = (a.power == 1.0) ? tk : pow(tk, a.power);
-        out[k] = (float)(dlo + (dhi - dlo) * tp);
-      }
-    } else if (l == 0) {
-      int nf = a.K, nodes = 0;
-      float fxc = 0.f, finv = 0.f, fa0 = 0.f;
-      const double k02 = a.k0 * a.k0;
-      const double alo = k02 * dlo * (2.0 + dlo), ahi = k02 * dhi * (2.0 + dhi);
-      const double ac = 0.5 * (alo + ahi), ah = 0.5 * (ahi - alo), amax = fmax(fabs(alo), fabs(ahi));
-      // (a comparison with a NaN is false: such slices keep the K references)
-      if (a.use_nodes && ah >= 0.0 && amax <= a.qmin * 0.125 && dlo > -0.5) {
-        const int n = wpm_node_count(ah, amax, a.qmin, a.k0, a.dz, min(kWpmMaxNodes, a.K - 1));
-        if (n > 0) {
-          nf = n;
-          nodes = 1;
-          fxc = (float)(ac / k02);
-          finv = ah > 0.0 ? (float)(k02 / ah) : 0.f;
-          const int c = n >> 1;   // the node nearest the centre
-          double tau[kWpmMaxNodes];
-          for (int j = 0; j < n; ++j) {
-            const int m = j == 0 ? c : (j <= c ? j - 1 : j);
-            tau[j] = (2 * m + 1 == n) ? 0.0 : cos((2 * m + 1) * M_PI / (2.0 * n));
-          }
-          fa0 = (float)(ac + ah * tau[0]);
-          for (int j = 0; j < n; ++j) {
-            double p = 1.0;
-            int i = 0;
-            for (int m = 0; m < n; ++m) {
-              if (m == j) continue;
-              p *= tau[j] - tau[m];
-              a.rec[row].other[j][i++] = (float)tau[m];
-            }
-            a.rec[row].da[j] = (float)(ah * (tau[j] - tau[0]));
-            a.rec[row].bw[j] = (float)(1.0 / p);
-          }
-        }
-      }
-      WpmSlice& r = a.rec[row];
-      r.nf = nf;
-      r.nodes = nodes;
-      r.xc = fxc;
-      r.inv_xh = finv;
-      r.a0 = fa0;
-      r.dlo = (float)dlo;
-      r.inv_range = dhi > dlo ? (float)(1.0 / (dhi - dlo)) : 0.f;
-    }
-  }
-  cl.sync();   // the shares stay readable until the first CTA has them
 }
 
 // ---------------------------------------------------------------------------
