@@ -217,12 +217,19 @@ int wpm_row_occupancy(int n, int e, int k, int K) { WAP_DISPATCH_INT(wrowocc, n,
 
 bool size_supported(int n) { return n >= 32 && n <= 2048 && (n & (n - 1)) == 0; }
 
-// rows per row-type CTA: fill kRowThreads, at most the grid height
-int rows_per_cta(int nx, int e, int ny) {
+// A pass of fewer CTAs than this takes smaller ones (64^2, one probe, 16 elements
+// per thread: one CTA, 8.2 us a slice; now 16 CTAs, 5.3).  Larger passes keep the
+// tuned shapes: splitting the 128 CTAs of one 512^2 probe cost 10 %.
+constexpr int kFewCtas = 128;
+
+// rows per row-type CTA: fill kRowThreads, at most the grid height; fewer, down to
+// two warps, where the pass has few CTAs
+int rows_per_cta(int nx, int e, int ny, int nb) {
   const int T = nx / e;
   int rows = kRowThreads / T;
   if (rows < 1) rows = 1;
   if (rows > ny) rows = ny;
+  while (rows > 1 && rows * T > 64 && (long long)(ny / rows) * nb < kFewCtas) rows >>= 1;
   return rows;
 }
 
@@ -370,8 +377,13 @@ int wap_plan_create(wap_plan** out, int ny, int nx, int max_batch, int op, int n
   p->max_batch = max_batch;
   p->op = op;
   p->n_bins = op == WAP_OP_WPM ? n_bins : 0;
-  p->row_e = nx >= 64 ? 16 : 8;
-  p->col_e = ny >= 64 ? 16 : 8;
+  // elements per thread where no tuned shape is set: plans of one or two Fresnel /
+  // AS probes take short chains (as tuned: 8 along rows, 4 along columns up to 256
+  // points), larger batches 16 from 128 points on
+  const bool few = op == WAP_OP_FRESNEL_AS && max_batch <= 2;
+  auto elems = [&](int n, bool col) { return few ? (n > 1024 ? 16 : col && n <= 256 ? 4 : 8) : n >= 128 ? 16 : 8; };
+  p->row_e = elems(nx, false);
+  p->col_e = elems(ny, true);
   p->col_w = default_col_w(ny, p->col_e, nx);
   p->generic = generic;
   int rc = generic ? generic_axis_create(&p->gen_x, nx, op == WAP_OP_WPM) : upload_twiddles(p);
@@ -534,7 +546,7 @@ static double col_bytes(const wap_plan* p, const ColArgs& c, int n_probes) {
 
 // batch chunks of at most 65535 probes (grid.y limit)
 cudaError_t row_chunks(const wap_plan* p, RowArgs r, int n_probes, cudaStream_t st) {
-  const int rows = rows_per_cta(p->nx, p->row_e, p->ny);
+  const int rows = rows_per_cta(p->nx, p->row_e, p->ny, n_probes);
   const ProfToken tok = prof_begin(WAP_KIND_ROW, st);
   for (int b0 = 0; b0 < n_probes; b0 += 65535) {
     r.probe0 = b0;
@@ -546,10 +558,14 @@ cudaError_t row_chunks(const wap_plan* p, RowArgs r, int n_probes, cudaStream_t 
 }
 
 cudaError_t col_chunks(const wap_plan* p, ColArgs c, int n_probes, cudaStream_t st) {
+  // few CTAs: fewer columns, down to four (32-byte row segments) and two warps
+  const int T = p->ny / p->col_e;
+  int w = p->col_w;
+  while (w > 4 && w * T > 64 && (long long)(p->nx / w) * n_probes < kFewCtas) w >>= 1;
   const ProfToken tok = prof_begin(WAP_KIND_COL, st);
   for (int b0 = 0; b0 < n_probes; b0 += 65535) {
     c.probe0 = b0;
-    cudaError_t e = launch_col(p->ny, p->col_e, c, std::min(65535, n_probes - b0), p->col_w, st);
+    cudaError_t e = launch_col(p->ny, p->col_e, c, std::min(65535, n_probes - b0), w, st);
     if (e != cudaSuccess) return e;
   }
   prof_end(tok, st, col_bytes(p, c, n_probes));

@@ -169,12 +169,14 @@ static cudaError_t chain_launch(int n, int e, const ChainArgs& a, cudaStream_t s
 constexpr int kChainMaxProbes = 2;
 
 // The chain pays one grid-wide barrier per pass (about two microseconds) in
-// place of a launch; measured on B200 it wins where the per-pass chain is
-// bound by the host's launch rate (up to 256^2: C1 0.18 vs 0.23 ms per call)
-// and loses on larger grids (1024^2 x 100 slices: 3.58 vs 2.69 ms), so by
-// default it serves grids up to kChainMaxSize.  WAP_KNOB_CHAIN: 0 off, 1 the
-// default, 4 / 8 / 16 that many elements per thread on any chain size.
-constexpr int kChainMaxSize = 256;
+// place of a launch.  Since the passes read and write their columns directly and
+// load their tables before the dependent-launch wait, launching each pass is the
+// faster way from 256^2 on (one probe, 20 slices, per call: 144 us in 41 launches,
+// 218 us as a chain; 1024^2 x 100 slices 2.6 against 3.6 ms).  At 128^2 it stands
+// in for the cluster kernel where the device refuses that; with the cluster kernel
+// switched off (WAP_KNOB_CLUSTER = 0) it serves up to 256^2.  WAP_KNOB_CHAIN: 0
+// off, 1 the default, 4 / 8 / 16 that many elements per thread on any chain size.
+static int chain_max_size() { return knob_value(WAP_KNOB_CLUSTER) == 0 ? 256 : 128; }
 
 int chain_forward(wap_plan* p, const RowArgs& r, const ColArgs& c, int n_probes, int n_slices, float2* stack,
                   cudaStream_t st) {
@@ -182,7 +184,7 @@ int chain_forward(wap_plan* p, const RowArgs& r, const ColArgs& c, int n_probes,
   const int kv = knob_value(WAP_KNOB_CHAIN);
   if (kv == 0) return -1;
   if (p->generic || p->ny != n || n < 128 || n > 2048 || n_probes > kChainMaxProbes) return -1;
-  if (kv < 2 && n > kChainMaxSize) return -1;
+  if (kv < 2 && n > chain_max_size()) return -1;
   cudaError_t e;
   int E = chain_elems(n);
   if (kv == 4 || kv == 8 || kv == 16) E = kv;

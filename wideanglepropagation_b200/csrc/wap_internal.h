@@ -96,7 +96,7 @@ const char* last_error();
 
 int check_common(const wap_plan* p, const float* V, int n_slices, int n_draws, const float* psi0, int n_probes,
                  float* exit);
-int rows_per_cta(int nx, int e, int ny);
+int rows_per_cta(int nx, int e, int ny, int nb);
 bool size_supported(int n);
 
 struct RowArgs;

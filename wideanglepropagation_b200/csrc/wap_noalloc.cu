@@ -144,7 +144,7 @@ extern "C" int wap_multislice_fwd_noalloc(const float* V, int n_slices, int ny, 
   int col_w = 16;
   while (col_w > 1 && (col_w * (ny / col_e) > kColThreads || (size_t)ny * col_w * 8 > 96 * 1024)) col_w >>= 1;
   if (col_w > nx) col_w = nx;
-  const int rows = rows_per_cta(nx, row_e, ny);
+  const int rows = rows_per_cta(nx, row_e, ny, n_probes);
   for (int s = 0; s <= n_slices; ++s) {
     r.slice = s;
     r.flags = (s == 0 ? ROW_LOAD_SRC : ROW_IFFT) | (s < n_slices ? (ROW_TRANS | ROW_FFT) : 0);

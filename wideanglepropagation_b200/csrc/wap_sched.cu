@@ -1749,7 +1749,7 @@ int wap_scan_grad_backward_ex(wap_scan* s, const float* grad_dp, const float* gr
       const int nb = std::min(65535, c.n_probes - b0);
       r.probe0 = b0;
       cc.probe0 = b0;
-      if ((e = launch_row(n, E, r, nb, rows_per_cta(n, E, n), st)) != cudaSuccess) return cuda_fail(e, "exit seed rows");
+      if ((e = launch_row(n, E, r, nb, rows_per_cta(n, E, n, nb), st)) != cudaSuccess) return cuda_fail(e, "exit seed rows");
       if ((e = launch_col(n, E, cc, nb, col_w, st)) != cudaSuccess) return cuda_fail(e, "exit seed columns");
     }
     sc.seed_add = sc.work;

@@ -419,7 +419,7 @@ static int reference_slices(const wap_plan* p, const Physics& ph, const float* V
                             WpmRowArgs w, int n_slices, int b0, int nb, float2* exit, float2* stack, cudaStream_t st) {
   const int K = p->n_bins;
   const long long plane = (long long)p->ny * p->nx;
-  const int rows = rows_per_cta(p->nx, p->row_e, p->ny);
+  const int rows = rows_per_cta(p->nx, p->row_e, p->ny, 65535);   // the bin split below fills the chip
   cudaError_t e;
   // Few probes leave most SMs idle (a 512^2 probe is 128 column and 128 row
   // CTAs): then the K bins are split across CTA groups - each column CTA
@@ -566,7 +566,6 @@ extern "C" int wap_wpm_fwd(wap_plan* p, const float* V, int n_slices, int n_draw
   w.ri_a = (float)ph.ri_a;
   w.ri_inv_den = (float)ph.ri_inv_den;
   w.snap_bstride = (long long)n_slices * plane;
-  const int rows = rows_per_cta(p->nx, p->row_e, p->ny);
 
   if (p->generic)
     return generic_wpm_forward(p, c, w, nodes, power_spacing, r.src, r.src_bstride, positions, n_slices, n_probes, dp,
