@@ -1,7 +1,10 @@
 """Pass launch shapes of small grids and few probes (fewer rows and columns per
-block, plans without a tuned shape) against the FP64 oracle.
+block, plans without a tuned shape), and the counts on either side of the
+hand-over to the persistent scheduler, against the FP64 oracle.
 
-Bar: rel-L2 <= 1e-5, as on the other paths.
+Bar: rel-L2 <= 1e-5, as on the other paths; probes on the two sides of the
+hand-over agree to 8e-6 (the scheduler's stage twiddles are float32 up to 160
+slices: at most 4.9e-6 from FP64 there, the passes 2.4e-6).
 """
 import numpy as np
 import pytest
@@ -41,3 +44,18 @@ def test_shapes_match_oracle(wap, ny, nx, B):
         ref = O.simulate_fresnel_as(V, O.move_probe(probe, tuple(pos[b])), H, dz, E)
         for g, r in zip((ex, dp, st), ref):
             assert O.rel_l2(g[b].cpu().numpy(), r) < TOL
+
+
+@pytest.mark.parametrize("n", [128, 256])
+def test_scheduler_hand_over(wap, n):
+    from wideanglepropagation_b200.propagation import SCAN_FROM_PROBES
+    V, probe, ps, dz, E = _case(n, n, 6)
+    H = wap.angular_spectrum_propagation_kernel(n, n, (ps, ps), dz, E)
+    many = SCAN_FROM_PROBES[n]
+    pos = np.random.default_rng(n).integers(0, n, (many, 2)).astype(np.int32)
+    out = []
+    for B in (many - 1, many):   # passes, scheduler
+        ex, dp, _ = wap.simulate_fresnel_as(V, probe, H, dz, E, positions=pos[:B], return_wavefronts=False)
+        out.append((ex[:many - 1], dp[:many - 1]))
+    for a, b in zip(*out):
+        assert float((a - b).norm() / b.norm()) < 8e-6

@@ -24,8 +24,8 @@ import ctypes
 import threading
 
 from . import _lib
-from .propagation import (SCAN_MIN_PROBES, SCAN_SIZES, StreamOrder, _detector, _device, _dp_shape, _prepare, _ptr,
-                          get_plan, scan_class, split_transfer)
+from .propagation import (SCAN_GRAD_FROM_PROBES, SCAN_MIN_PROBES, StreamOrder, _detector, _device,  # noqa: F401
+                          _dp_shape, _prepare, _ptr, get_plan, scan_class, split_transfer)
 
 # gradient scans (persistent scheduler) by shape, each with the StreamOrder of
 # its workspace; a scan is held from the forward until its backward has run,
@@ -96,7 +96,7 @@ class MultisliceFunction(torch.autograd.Function):
         Vc, psi, per_probe, pos, dr, B, N, ny, nx, batched = _prepare(V.detach(), probe, positions, draw, dev)
         Hc, Hl = split_transfer(H, dev)
         ctx.scan = None
-        if ctx.needs_input_grad[0] and ny == nx and ny in SCAN_SIZES and B >= SCAN_MIN_PROBES and not per_probe:
+        if ctx.needs_input_grad[0] and ny == nx and B >= SCAN_GRAD_FROM_PROBES.get(ny, B + 1) and not per_probe:
             # persistent scheduler: forward with checkpoints now, adjoint later
             exit_wave = torch.empty((B, ny, nx), dtype=torch.complex64, device=dev)
             dp = torch.empty(_dp_shape(B, ny, nx, det), dtype=torch.float32, device=dev)

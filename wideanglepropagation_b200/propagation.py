@@ -437,10 +437,17 @@ def _prepare(potential, probe, positions, draw, dev):
     return V, psi, per_probe, pos, dr, B, n_slices, ny, nx, batched
 
 
-SCAN_SIZES = (128, 256, 512, 1024)
 SCAN_MIN_PROBES = 8
-# forwards of at most this many probes on these square grids run as one launch (a
-# cooperative grid, or a thread-block cluster per probe at 128)
+# Probes from which the persistent scheduler is the faster way on each grid: a step
+# of few small waves is a chain of hand-overs between its CTAs, 17 us a slice
+# whatever the count, where the pass kernels take 5 to 20.  Measured, 40 slices,
+# scheduler / passes: 16 probes on 128^2 0.69 / 0.34 ms, 32 on 256^2 0.85 / 0.94,
+# 16 on 256^2 0.83 / 0.61, 8 on 512^2 1.07 / 1.33.  With the gradient (32 slices):
+# 32 on 128^2 1.81 / 1.23, 16 on 256^2 1.98 / 1.86, 32 on 256^2 2.05 / 3.15.
+SCAN_FROM_PROBES = {128: 64, 256: 28, 512: 8, 1024: 8}
+SCAN_GRAD_FROM_PROBES = {128: 64, 256: 18, 512: 8, 1024: 8}
+# forwards of at most this many probes on these square grids may run as one launch (a
+# thread-block cluster per probe at 128, a cooperative grid where that is not to be had)
 CHAIN_SIZES = (128, 256)
 CHAIN_MAX_PROBES = 2
 _scans: dict = {}          # key -> (scan handle, StreamOrder)
@@ -607,11 +614,10 @@ def simulate_fresnel_as(potential, probe, prop_kernel, slice_thickness, energy, 
     (``accumulate_patterns``), e.g. the frozen-phonon draws of each scan
     position into one float32 pattern per position; exit waves stay per probe.
 
-    Calls that run on the persistent scheduler (many probes of one probe) or
-    as one cooperative launch (one or two probes on a square 256 grid; on a
-    128 grid they run as one thread-block cluster per probe, without
-    device-side waits) raise WapError if one of their bounded device-side
-    waits expired; with
+    Calls that run on the persistent scheduler (many probes of one probe) or as one
+    cooperative launch (one or two probes on a square 128 grid where the device
+    refuses the thread-block cluster that usually serves them) raise WapError if
+    one of their bounded device-side waits expired; with
     ``check=False`` the call returns without waiting for the GPU and the
     failure is raised by ``check_errors()`` or by a later call.
     """
@@ -626,7 +632,7 @@ def simulate_fresnel_as(potential, probe, prop_kernel, slice_thickness, energy, 
     det = _detector((ny, nx), sampling, energy, max_angle, parity)
     exit_wave = torch.empty((B, ny, nx), dtype=torch.complex64, device=dev)
     dp = torch.empty(_dp_shape(B, ny, nx, det), dtype=torch.float32, device=dev)
-    if (not return_wavefronts and ny == nx and ny in SCAN_SIZES and B >= SCAN_MIN_PROBES
+    if (not return_wavefronts and ny == nx and B >= SCAN_FROM_PROBES.get(ny, B + 1)
             and not per_probe):
         # many probes of one shared probe: the persistent batched scheduler
         _scan_run(V, psi, pos, dr, H, H_lo, slice_thickness, energy, exit_wave, dp, det, check=check)
