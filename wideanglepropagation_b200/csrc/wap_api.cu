@@ -668,8 +668,10 @@ int fresnel_forward(wap_plan* p, const float* V, int n_slices, int n_draws, cons
     if (rc2 != -1) return rc2;
   }
 
+  c.h_ready = 1;   // the first row pass waits for all that came before this call
   for (int s = 0; s <= n_slices; ++s) {
     r.slice = s;
+    r.tab_ready = s > 0;
     r.flags = (s == 0 ? ROW_LOAD_SRC : ROW_IFFT) | (s < n_slices ? (trans_flag | ROW_FFT) : 0);
     r.snap = nullptr;
     if (stack && s >= 1) {

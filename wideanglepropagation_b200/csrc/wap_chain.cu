@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(kChainThreads, 2) chain_kernel(const ChainArgs
   const int cblocks = N / (kChainThreads / T);   // column tiles per probe
   const int runits = rblocks * a.n_probes, cunits = cblocks * a.n_probes;
   const int tflag = r.ttab ? ROW_TRANS_TAB : ROW_TRANS;
+  float2 pre0[early_elems<E>()], pre1[early_elems<E>()];
   unsigned k = 0;
   for (int s = 0; s <= a.n_slices; ++s) {
     r.slice = s;
@@ -91,14 +92,14 @@ __global__ void __launch_bounds__(kChainThreads, 2) chain_kernel(const ChainArgs
     r.snap = (a.stack && s >= 1) ? a.stack + (long long)(s - 1) * plane : nullptr;
     r.snap_bstride = (long long)a.n_slices * plane;
     for (int u = blockIdx.x; u < runits; u += gridDim.x) {
-      row_pass_body<N, E>(r, tw, buf, u % rblocks, u / rblocks);
+      row_pass_body<N, E>(r, tw, buf, u % rblocks, u / rblocks, pre0, false);
       __syncthreads();
     }
     if (s == a.n_slices) break;
     if (!chain_barrier(a, ++k)) return;
     c.flags = (s == a.n_slices - 1 && c.dp) ? COL_DP : 0;
     for (int u = blockIdx.x; u < cunits; u += gridDim.x) {
-      col_pass_body<N, E, false>(c, tw, buf, u % cblocks, u / cblocks);
+      col_pass_body<N, E, false>(c, tw, buf, u % cblocks, u / cblocks, pre0, pre1, false);
       __syncthreads();
     }
     if (!chain_barrier(a, ++k)) return;

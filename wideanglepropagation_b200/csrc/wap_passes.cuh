@@ -80,6 +80,7 @@ struct RowArgs {
   float e_plus_e0;           // E + E0 (for dn/dV)
   int tw_ready;              // tw was not written by a kernel of this stream (a plan's
                              // table): read before the programmatic-launch wait
+  int tab_ready;             // ttab was complete two launches ago: likewise
 };
 
 struct ColArgs {
@@ -98,6 +99,8 @@ struct ColArgs {
   int probe0;
   float seed_scale;          // n_px
   int tw_ready;              // as RowArgs::tw_ready
+  int h_ready;               // H was complete two launches ago (passes of a forward): read
+                             // before the programmatic-launch wait
 };
 
 // numpy.fft.fftfreq(n, d)[i] in float64: i * (1/(n d)) with the upper half
@@ -196,11 +199,31 @@ struct RowCfg {
   static constexpr int PADN = RowExchange<true>::padded(NX);
 };
 
+// Short-chain shapes (E <= 8, the launches of few probes) fetch the transmission
+// row (the transfer function, in the column pass) into registers ahead of the
+// transforms; E = 16 keeps the registers.
+template <int E>
+__host__ __device__ constexpr int early_elems() { return E <= 8 ? E : 1; }
+
+// this thread's elements of the transmission row, read through L2
+template <int NX, int E>
+__device__ __forceinline__ void row_fetch_t(const RowArgs& a, int bx, int by, float2 (&tpre)[early_elems<E>()]) {
+  constexpr int T = RowCfg<NX, E>::T;
+  const int rl = threadIdx.x / T, t = threadIdx.x - rl * T;
+  const int row = bx * (blockDim.x / T) + rl, b = a.probe0 + by;
+  const int d = a.draw ? a.draw[b] : 0;
+  const float2* trow = a.ttab + (long long)d * a.v_draw_stride + ((long long)a.slice * a.ny + row) * NX;
+#pragma unroll
+  for (int e = 0; e < early_elems<E>(); ++e) tpre[e] = __ldcg(trow + t + T * e);
+}
+
 // One row tile (rows blockDim.x / T consecutive rows of probe probe0 + by):
 // the body of row_pass_kernel and of the single-probe chain kernel.  tw is
-// the twiddle table in shared memory, xbuf the exchange buffer.
+// the twiddle table in shared memory, xbuf the exchange buffer; fetched: tpre
+// holds the transmission row already.
 template <int NX, int E>
-__device__ __forceinline__ void row_pass_body(const RowArgs& a, const float4* tw, float2* xbuf, int bx, int by) {
+__device__ __forceinline__ void row_pass_body(const RowArgs& a, const float4* tw, float2* xbuf, int bx, int by,
+                                              float2 (&tpre)[early_elems<E>()], bool fetched) {
   using C = RowCfg<NX, E>;
   constexpr int T = C::T;
   const int rows = blockDim.x / T;
@@ -237,17 +260,8 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a, const float4* tw
 #pragma unroll
     for (int e = 0; e < E; ++e) v[e] = __ldcg(prow + t + T * e);
   }
-  // Short-chain shapes (E <= 8, the single-probe launches) fetch the
-  // transmission row before the inverse transform, so its L2 latency overlaps
-  // the transform instead of following it; E = 16 keeps the registers.
   constexpr bool kEarlyT = E <= 8;
-  float2 tpre[kEarlyT ? E : 1];
-  if (kEarlyT && (f & ROW_TRANS_TAB)) {
-    const int d = a.draw ? a.draw[b] : 0;
-    const float2* trow = a.ttab + (long long)d * a.v_draw_stride + (long long)a.slice * plane + (long long)row * NX;
-#pragma unroll
-    for (int e = 0; e < (kEarlyT ? E : 1); ++e) tpre[e] = __ldg(trow + t + T * e);
-  }
+  if (kEarlyT && (f & ROW_TRANS_TAB) && !fetched) row_fetch_t<NX, E>(a, bx, by, tpre);
 
   if (f & ROW_IFFT) {
     fft<NX, E, true>(v, t, xs, tw);
@@ -264,7 +278,7 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a, const float4* tw
   if (f & ROW_TRANS_TAB) {
     if constexpr (kEarlyT) {
 #pragma unroll
-      for (int e = 0; e < E; ++e) v[e] = cmul(v[e], tpre[e]);
+      for (int e = 0; e < early_elems<E>(); ++e) v[e] = cmul(v[e], tpre[e]);
     } else {
       const int d = a.draw ? a.draw[b] : 0;
       const float2* trow = a.ttab + (long long)d * a.v_draw_stride + (long long)a.slice * plane + (long long)row * NX;
@@ -328,11 +342,17 @@ row_pass_kernel(const RowArgs a) {
   // its tail (one L2 round trip less on the chain of a single probe)
   if (a.tw_ready)
     for (int i = threadIdx.x; i < C::P::TW_SIZE; i += blockDim.x) tw[i] = __ldg(a.tw + i);
+  // and from the second slice on the transmission table is complete before this
+  // launch (the first row pass has waited for the kernel that writes it): its row,
+  // which comes from HBM, arrives under the previous pass's tail
+  float2 tpre[early_elems<E>()];
+  const bool fetch = E <= 8 && a.tab_ready && (a.flags & ROW_TRANS_TAB);
+  if (fetch) row_fetch_t<NX, E>(a, blockIdx.x, blockIdx.y, tpre);
   pdl_wait_then_release();
   if (!a.tw_ready)
     for (int i = threadIdx.x; i < C::P::TW_SIZE; i += blockDim.x) tw[i] = a.tw[i];
   __syncthreads();
-  row_pass_body<NX, E>(a, tw, xbuf, blockIdx.x, blockIdx.y);
+  row_pass_body<NX, E>(a, tw, xbuf, blockIdx.x, blockIdx.y, tpre, fetch);
 }
 
 // ----------------------------------------------------------------------------
@@ -356,10 +376,27 @@ __device__ __forceinline__ void tile_load(float2* tile, const float2* __restrict
 // ----------------------------------------------------------------------------
 // column pass
 // ----------------------------------------------------------------------------
+// this thread's elements of H (hi and lo parts)
+template <int NY, int E>
+__device__ __forceinline__ void col_fetch_h(const ColArgs& a, int bx, float2 (&hpre)[early_elems<E>()],
+                                            float2 (&lpre)[early_elems<E>()]) {
+  constexpr int T = FFTPlan<NY, E>::T;
+  const int W = blockDim.x / T, t = threadIdx.x / W, col = bx * W + threadIdx.x % W;
+#pragma unroll
+  for (int e = 0; e < early_elems<E>(); ++e) {
+    const long long o = (long long)(t + T * e) * a.nx + col;
+    hpre[e] = __ldg(a.H + o);
+    lpre[e] = a.H_lo ? __ldg(a.H_lo + o) : make_float2(0.f, 0.f);
+  }
+}
+
 // One column tile (W = blockDim.x / T columns of probe probe0 + by): the body
-// of col_pass_kernel and of the single-probe chain kernel.
+// of col_pass_kernel and of the single-probe chain kernel; fetched: hpre, lpre
+// hold the transfer function already.
 template <int NY, int E, bool SEED>
-__device__ __forceinline__ void col_pass_body(const ColArgs& a, const float4* tw, float2* tile, int bx, int by) {
+__device__ __forceinline__ void col_pass_body(const ColArgs& a, const float4* tw, float2* tile, int bx, int by,
+                                              float2 (&hpre)[early_elems<E>()], float2 (&lpre)[early_elems<E>()],
+                                              bool fetched) {
   using P = FFTPlan<NY, E>;
   constexpr int T = P::T;
   const int W = blockDim.x / T;
@@ -378,18 +415,8 @@ __device__ __forceinline__ void col_pass_body(const ColArgs& a, const float4* tw
   float2 v[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) v[e] = __ldcg(pcol + (long long)(t + T * e) * nx);
-  // short-chain shapes fetch H (hi and lo) before the forward transform, as
-  // the row pass does with the transmission
   constexpr bool kEarlyH = E <= 8;
-  float2 hpre[kEarlyH ? E : 1], lpre[kEarlyH ? E : 1];
-  if (kEarlyH && !(f & COL_NO_H)) {
-#pragma unroll
-    for (int e = 0; e < (kEarlyH ? E : 1); ++e) {
-      const long long o = (long long)(t + T * e) * nx + col;
-      hpre[e] = __ldg(a.H + o);
-      lpre[e] = a.H_lo ? __ldg(a.H_lo + o) : make_float2(0.f, 0.f);
-    }
-  }
+  if (kEarlyH && !(f & COL_NO_H) && !fetched) col_fetch_h<NY, E>(a, bx, hpre, lpre);
 
   if (!(f & COL_NO_FFT)) fft<NY, E, false>(v, t, xs, tw);
 
@@ -423,10 +450,10 @@ __device__ __forceinline__ void col_pass_body(const ColArgs& a, const float4* tw
   if (kEarlyH && !(f & COL_NO_H)) {
     if (f & COL_CONJ_H) {
 #pragma unroll
-      for (int e = 0; e < E; ++e) v[e] = cmulc_hl(v[e], hpre[e], lpre[e]);
+      for (int e = 0; e < early_elems<E>(); ++e) v[e] = cmulc_hl(v[e], hpre[e], lpre[e]);
     } else {
 #pragma unroll
-      for (int e = 0; e < E; ++e) v[e] = cmul_hl(v[e], hpre[e], lpre[e]);
+      for (int e = 0; e < early_elems<E>(); ++e) v[e] = cmul_hl(v[e], hpre[e], lpre[e]);
     }
   } else if (!(f & COL_NO_H)) {
     const float2* hcol = a.H + col;
@@ -479,11 +506,14 @@ col_pass_kernel(const ColArgs a) {
   float2* tile = reinterpret_cast<float2*>(tw + P::TW_SIZE);
   if (a.tw_ready)
     for (int i = threadIdx.x; i < P::TW_SIZE; i += blockDim.x) tw[i] = __ldg(a.tw + i);
+  float2 hpre[early_elems<E>()], lpre[early_elems<E>()];
+  const bool fetch = E <= 8 && a.h_ready && !(a.flags & COL_NO_H);
+  if (fetch) col_fetch_h<NY, E>(a, blockIdx.x, hpre, lpre);
   pdl_wait_then_release();
   if (!a.tw_ready)
     for (int i = threadIdx.x; i < P::TW_SIZE; i += blockDim.x) tw[i] = a.tw[i];
   __syncthreads();
-  col_pass_body<NY, E, SEED>(a, tw, tile, blockIdx.x, blockIdx.y);
+  col_pass_body<NY, E, SEED>(a, tw, tile, blockIdx.x, blockIdx.y, hpre, lpre, fetch);
 }
 
 // The WPM bin propagator applied to v = X * Hvac by the direct formulas, for
