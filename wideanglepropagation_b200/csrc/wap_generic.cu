@@ -36,6 +36,14 @@ __global__ void __launch_bounds__(BLUE ? kGenThreads : 2 * kGenThreads, BLUE ? 3
   const int b = a.probe0 + blockIdx.y;
   GenRowOp op = gen_row_op(a, b, row);
   const MixMem mem{bufs + min(rl, rows - 1) * ax.m, rows * ax.m, 1};
+  if (a.fetch) {
+    // the rows' transmission under the previous pass's tail
+    float2* ts = bufs + 2 * rows * ax.m;
+    const int row0 = blockIdx.x * rows, count = min(rows, a.ny - row0) * a.nx;
+    const float2* src = op.trow + (row0 - row) * a.nx;
+    for (int i = threadIdx.x; i < count; i += blockDim.x) ts[i] = __ldcg(src + i);
+    op.trow = ts + rl * a.nx;
+  }
   __syncthreads();
   pdl_wait_then_release();
   mix_pass<BLUE>(ax, (a.flags & (ROW_IFFT | ROW_FFT)) == (ROW_IFFT | ROW_FFT) ? 2 : 1, tw, mem, t, live, op);
@@ -53,6 +61,19 @@ __global__ void __launch_bounds__(2 * kGenThreads, 2) gen_col_kernel(const GenCo
   const int b = a.probe0 + blockIdx.y;
   GenColOp op = gen_col_op(a, b, col);
   const MixMem mem{bufs + c, ax.m * w, w};
+  if (a.fetch) {   // H, an input of the call, under the previous pass's tail
+    float4* hs = reinterpret_cast<float4*>(bufs + 2 * ax.m * w);
+    const int cols = min(w, a.nx - (int)blockIdx.x * w);
+    for (int i = threadIdx.x; i < a.ny * w; i += blockDim.x) {
+      const int r = i / w, k = i & (w - 1);
+      if (k < cols) {
+        const int o = r * a.nx + blockIdx.x * w + k;
+        const float2 h = __ldg(a.H + o), l = a.H_lo ? __ldg(a.H_lo + o) : make_float2(0.f, 0.f);
+        hs[i] = make_float4(h.x, h.y, l.x, l.y);
+      }
+    }
+    op.hq = hs + c;
+  }
   __syncthreads();
   pdl_wait_then_release();
   mix_pass<false>(ax, 2, tw, mem, t, live, op);
@@ -71,14 +92,19 @@ __global__ void __launch_bounds__(256) gen_trans_table_kernel(const float* __res
 cudaError_t launch_gen_row(GenRowArgs& a, int nb, cudaStream_t st) {
   if (a.ax.pow2) return launch_blue_row(a, nb, st);
   a.rows = gen_lines(a.ny, a.ax.threads, 64, std::max(1, 32 / a.ax.threads), kGenThreads, nb);
-  const size_t smem = a.ax.tw_len * sizeof(float4) + 2 * (size_t)a.rows * a.ax.m * sizeof(float2);
-  return launch_gen(a.ax.blue ? gen_row_kernel<true> : gen_row_kernel<false>, dim3((a.ny + a.rows - 1) / a.rows, nb), a.rows * a.ax.threads, smem, st, a);
+  a.fetch = a.tab_ready && (a.flags & ROW_TRANS_TAB) && gen_fetch(a.ax, (long long)a.ny * nb);
+  const size_t smem =
+      a.ax.tw_len * sizeof(float4) + (size_t)a.rows * (2 * a.ax.m + (a.fetch ? a.nx : 0)) * sizeof(float2);
+  return launch_gen(a.ax.blue ? gen_row_kernel<true> : gen_row_kernel<false>, dim3((a.ny + a.rows - 1) / a.rows, nb),
+                    a.rows * a.ax.threads, smem, st, a);
 }
 
 static cudaError_t launch_gen_col(GenColArgs& a, int nb, cudaStream_t st) {
   if (a.ax.pow2) return launch_blue_col(a, nb, st);
   a.w = gen_cols(a.ax, a.nx, nb);
-  const size_t smem = a.ax.tw_len * sizeof(float4) + 2 * (size_t)a.ax.m * a.w * sizeof(float2);
+  a.fetch = gen_fetch(a.ax, (long long)a.nx * nb);
+  const size_t smem = a.ax.tw_len * sizeof(float4) +
+                      (size_t)a.w * (2 * a.ax.m * sizeof(float2) + (a.fetch ? a.ny * sizeof(float4) : 0));
   return launch_gen(gen_col_kernel, dim3((a.nx + a.w - 1) / a.w, nb), a.w * a.ax.threads, smem, st, a);
 }
 
@@ -296,6 +322,7 @@ int generic_fresnel_forward(wap_plan* p, const RowArgs& base, const ColArgs& cba
     r.probe0 = c.probe0 = b0;
     for (int s = 0; s <= n_slices; ++s) {
       r.slice = s;
+      r.tab_ready = s > 0;
       r.flags = (s == 0 ? ROW_LOAD_SRC : ROW_IFFT) | (s < n_slices ? (trans | ROW_FFT) : 0);
       r.snap = nullptr;
       if (stack && s >= 1) {

@@ -45,6 +45,8 @@ struct GenRowArgs {
   GenAxis ax;                 // along x
   int ny, nx, slice, flags, probe0;
   int rows;                   // per block
+  int tab_ready;              // ttab was complete two launches ago
+  int fetch;                  // its rows go to shared memory before the wait
   float2 scale;               // after the inverse row DFT, hi + lo
   float ri_a, ri_inv_den, kphase;
 };
@@ -62,12 +64,12 @@ struct GenRowOp {
   const float2* srow;
   float2* snap;
   const float* vrow;
-  const float2* trow;
+  const float2* trow;         // the row's table, or its copy in shared memory
   int sx, f;
   // the spatial value of the transformed line (or of the source) -> the value to transform
   __device__ __forceinline__ float2 slice_value(int p, float2 y) const {
     if (snap) __stcs(snap + p, y);
-    if (f & ROW_TRANS_TAB) y = cmul(y, __ldg(trow + p));
+    if (f & ROW_TRANS_TAB) y = cmul(y, trow[p]);
     else if (f & ROW_TRANS) y = cmul(y, gen_transmission(__ldg(vrow + p), a.ri_a, a.ri_inv_den, a.kphase));
     return y;
   }
@@ -126,6 +128,7 @@ struct GenColArgs {
   Detector det;
   GenAxis ax;                 // along y
   int ny, nx, w, flags, probe0;   // w: columns per block
+  int fetch;                  // H goes to shared memory before the wait
 };
 
 struct GenColOp {
@@ -133,12 +136,17 @@ struct GenColOp {
   float2* pcol;
   const float2* hcol;
   const float2* lcol;
+  const float4* hq;           // this column's (hi, lo) in shared memory, stride w, or null
   float* dp;
   int drx;
   __device__ __forceinline__ float2 load(int p) const { return __ldcg(pcol + p * a.nx); }
   __device__ __forceinline__ float2 turn(int p, float2 y) const {
-    const int o = p * a.nx;
-    y = lcol ? cmul_hl(y, __ldg(hcol + o), __ldg(lcol + o)) : cmul(y, __ldg(hcol + o));
+    if (hq) {
+      y = cmul_tw(y, hq[p * a.w]);
+    } else {
+      const int o = p * a.nx;
+      y = lcol ? cmul_hl(y, __ldg(hcol + o), __ldg(lcol + o)) : cmul(y, __ldg(hcol + o));
+    }
     if (dp) gen_pattern(dp, a.det, drx, p, a.ny, y);
     return cconj(y);
   }
@@ -150,6 +158,7 @@ __device__ __forceinline__ GenColOp gen_col_op(const GenColArgs& a, int b, int c
   op.pcol = a.psi + (long long)b * a.psi_bstride + col;
   op.hcol = a.H + col;
   op.lcol = a.H_lo ? a.H_lo + col : nullptr;
+  op.hq = nullptr;
   op.dp = (a.flags & COL_DP) ? a.dp + (long long)b * a.det.plane() : nullptr;
   op.drx = shifted(col, a.nx) - a.det.x0;
   return op;
@@ -191,6 +200,12 @@ inline float2 inverse_scale(long long plane) {
   const double s = 1.0 / (double)plane;
   return make_float2((float)s, (float)(s - (double)(float)s));
 }
+
+// Whether a pass of `lines` lines is short of threads (under half the chip's): then its
+// tables are copied to shared memory before the wait, off the chain of the pass
+// (100^2, 100 slices: 1.23 -> 0.98 ms); a fuller pass hides their latency and the
+// copy costs (1000^2, 20 slices: 1.24 -> 1.47 ms).
+inline bool gen_fetch(const GenAxis& ax, long long lines) { return lines * ax.threads <= 148LL * 1024; }
 
 cudaError_t launch_gen_row(GenRowArgs& a, int nb, cudaStream_t st);
 // Bluestein axes of Fresnel / AS plans (wap_bluestein.cu)
