@@ -359,7 +359,7 @@ int wap_plan_create(wap_plan** out, int ny, int nx, int max_batch, int op, int n
   if (!out) return fail(WAP_ERR_ARG, "plan pointer is NULL");
   *out = nullptr;
   // power-of-two grids in [32, 2048] take the fast path; a grid with another
-  // side (17 .. 1024) runs the Bluestein transforms of wap_generic.cu
+  // side (17 .. 1024) runs the mixed-radix or Bluestein transforms of wap_generic.cu
   const bool generic = !size_supported(ny) || !size_supported(nx);
   auto axis_ok = [](int n) { return size_supported(n) || generic_size_supported(n); };
   if (!axis_ok(ny) || !axis_ok(nx))
@@ -589,6 +589,10 @@ int build_trans_table(wap_plan* p, const float* V, int n_slices, int n_draws, co
   const size_t need = (size_t)n_draws * n_slices * p->ny * p->nx;
   cudaError_t e = cudaSuccess;
   if (need > p->ttab_cap) {
+    // a stream in capture may not allocate: the passes evaluate exp(i phi) inline
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)
+      return fail(WAP_ERR_CUDA, "transmission table: the stream is being captured");
     cudaFree(p->ttab);
     p->ttab = nullptr;
     p->ttab_cap = 0;
@@ -658,9 +662,9 @@ int fresnel_forward(wap_plan* p, const float* V, int n_slices, int n_draws, cons
   }
   if (p->generic)
     return generic_fresnel_forward(p, r, c, n_slices, n_probes, reinterpret_cast<float2*>(stack), st);
-  // few probes: every slice in one launch when the grid qualifies - the wave
-  // held in a thread-block cluster (wap_cluster.cu), else a cooperative grid
-  // (wap_chain.cu) - else one launch per pass below
+  // few probes on 128^2: every slice in one launch - the wave held in a thread-block
+  // cluster (wap_cluster.cu), else a cooperative grid (wap_chain.cu) - else one
+  // launch per pass below
   if (!ckpt) {
     int rc2 = cluster_forward(p, r, c, n_probes, n_slices, reinterpret_cast<float2*>(stack), st);
     if (rc2 != -1) return rc2;
