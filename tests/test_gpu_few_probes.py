@@ -33,7 +33,8 @@ def _case(ny, nx, N):
 
 
 @pytest.mark.parametrize("ny,nx,B", [(32, 32, 1), (64, 64, 1), (64, 64, 3), (32, 256, 1), (512, 128, 2), (2048, 32, 1),
-                                     (128, 64, 5), (256, 256, 1), (256, 256, 4)])
+                                     (128, 64, 5), (256, 256, 1), (256, 256, 4), (256, 256, 8), (128, 128, 16),
+                                     (256, 512, 6)])
 def test_shapes_match_oracle(wap, ny, nx, B):
     from oracle import propagation_oracle as O
     V, probe, ps, dz, E = _case(ny, nx, 4)

@@ -283,13 +283,17 @@ using namespace wap;
 // plan
 // ----------------------------------------------------------------------------
 static int upload_twiddles(wap_plan* p) {
-  for (int which = 0; which < 2; ++which) {
-    const int n = which == 0 ? p->nx : p->ny;
-    const int e = which == 0 ? p->row_e : p->col_e;
-    std::vector<float4> h = twiddle_table(n, e);
-    float4*& d = which == 0 ? p->tw_row : p->tw_col;
+  for (int which = 0; which < 4; ++which) {
+    const int n = which % 2 == 0 ? p->nx : p->ny;
+    int e = which % 2 == 0 ? p->row_e : p->col_e;
+    float4*& d = which == 0 ? p->tw_row : which == 1 ? p->tw_col : which == 2 ? p->tw_row8 : p->tw_col8;
     if (d) cudaFree(d);
     d = nullptr;
+    if (which >= 2) {
+      if (e != 16 || n < 128 || n > 1024) continue;
+      e = 8;
+    }
+    std::vector<float4> h = twiddle_table(n, e);
     cudaError_t err = cudaMalloc(&d, h.size() * sizeof(float4));
     if (err != cudaSuccess) return cuda_fail(err, "cudaMalloc(twiddles)");
     err = cudaMemcpy(d, h.data(), h.size() * sizeof(float4), cudaMemcpyHostToDevice);
@@ -324,6 +328,8 @@ static void plan_free(wap_plan* p) {
   if (!p) return;
   cudaFree(p->tw_row);
   cudaFree(p->tw_col);
+  cudaFree(p->tw_row8);
+  cudaFree(p->tw_col8);
   cudaFree(p->fields);
   cudaFree(p->dpbuf);
   cudaFree(p->blend);
@@ -545,12 +551,25 @@ static double col_bytes(const wap_plan* p, const ColArgs& c, int n_probes) {
 }
 
 // batch chunks of at most 65535 probes (grid.y limit)
+// A shape of 16 elements per thread was chosen for a full chip.  Passes of at most
+// kMediumRows pixels take 8 along the rows, of at most kMediumCols along the columns:
+// more and shorter threads.  Measured per slice (row e, column e, columns per CTA):
+// 16 probes on 256^2 15.5 -> 14.7 us, 4 on 512^2 20.6 -> 19.0, 8 on 256^2 11.6 -> 10.5
+// with 8 columns; 4 on 256^2 9.2 -> 8.1, 16 on 128^2 8.6 -> 7.0 with short columns too;
+// from 3 probes on 1024^2 on, 16 stays the faster (62.5 against 65.8).
+constexpr long long kMediumRows = 1LL << 20, kMediumTiles = 1LL << 19, kMediumCols = 1LL << 18;
+
 cudaError_t row_chunks(const wap_plan* p, RowArgs r, int n_probes, cudaStream_t st) {
-  const int rows = rows_per_cta(p->nx, p->row_e, p->ny, n_probes);
+  int elems = p->row_e;
+  if (p->tw_row8 && r.tw == p->tw_row && (long long)p->ny * p->nx * n_probes <= kMediumRows) {
+    elems = 8;
+    r.tw = p->tw_row8;
+  }
+  const int rows = rows_per_cta(p->nx, elems, p->ny, n_probes);
   const ProfToken tok = prof_begin(WAP_KIND_ROW, st);
   for (int b0 = 0; b0 < n_probes; b0 += 65535) {
     r.probe0 = b0;
-    cudaError_t e = launch_row(p->nx, p->row_e, r, std::min(65535, n_probes - b0), rows, st);
+    cudaError_t e = launch_row(p->nx, elems, r, std::min(65535, n_probes - b0), rows, st);
     if (e != cudaSuccess) return e;
   }
   prof_end(tok, st, row_bytes(p, r, n_probes));
@@ -559,13 +578,22 @@ cudaError_t row_chunks(const wap_plan* p, RowArgs r, int n_probes, cudaStream_t 
 
 cudaError_t col_chunks(const wap_plan* p, ColArgs c, int n_probes, cudaStream_t st) {
   // few CTAs: fewer columns, down to four (32-byte row segments) and two warps
-  const int T = p->ny / p->col_e;
-  int w = p->col_w;
+  const long long pixels = (long long)p->ny * p->nx * n_probes;
+  int elems = p->col_e, w = p->col_w;
+  if (p->tw_col8 && c.tw == p->tw_col && pixels <= kMediumTiles) {
+    w = std::min(w, 8);
+    if (pixels <= kMediumCols) {
+      elems = 8;
+      c.tw = p->tw_col8;
+      while (w > 1 && w * (p->ny / 8) > kColThreads) w >>= 1;
+    }
+  }
+  const int T = p->ny / elems;
   while (w > 4 && w * T > 64 && (long long)(p->nx / w) * n_probes < kFewCtas) w >>= 1;
   const ProfToken tok = prof_begin(WAP_KIND_COL, st);
   for (int b0 = 0; b0 < n_probes; b0 += 65535) {
     c.probe0 = b0;
-    cudaError_t e = launch_col(p->ny, p->col_e, c, std::min(65535, n_probes - b0), w, st);
+    cudaError_t e = launch_col(p->ny, elems, c, std::min(65535, n_probes - b0), w, st);
     if (e != cudaSuccess) return e;
   }
   prof_end(tok, st, col_bytes(p, c, n_probes));

@@ -1,5 +1,6 @@
 // One-launch multislice of a single probe (or two): every slice's row and
-// column pass in one cooperative kernel, separated by grid-wide barriers.
+// column pass in one cooperative kernel, separated by grid-wide barriers (the
+// stand-in for the cluster kernel on 128^2; see chain_max_size).
 //
 // A probe's pass is a few hundred CTAs and a few microseconds of work, so the
 // per-pass chain (2 N + 1 launches, programmatic dependent launch) is bound by

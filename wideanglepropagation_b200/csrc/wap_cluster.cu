@@ -26,7 +26,7 @@
 //
 // One cluster per probe.  Square grids of 128 points by default, 256 when
 // asked for through WAP_KNOB_CLUSTER (there the 16 SMs of one cluster take
-// longer than the cooperative chain on all SMs; a 512^2 wave would need
+// longer than a launch per pass on all SMs; a 512^2 wave would need
 // 128 KB of slab and 128 KB of column buffer per CTA).  Falls back (-1) when
 // the device cannot co-schedule a 16-CTA cluster of the kernel.
 #include <cuda_runtime.h>
@@ -286,7 +286,7 @@ int cluster_forward(wap_plan* p, const RowArgs& r, const ColArgs& c, int n_probe
   if (kv == 0) return -1;
   if (p->generic || p->ny != n || n_probes > kClusterMaxProbes || n_slices < 1) return -1;
   // by default 128^2 only: at 256^2 the 16 SMs of a cluster take longer than
-  // the cooperative chain on all SMs (B200, 20 slices: 164 vs 154 us)
+  // a launch per pass on all SMs (B200, 20 slices: 164 us against 144 per call)
   if (n != 128 && !(n == 256 && kv > 1)) return -1;
   int E = cluster_elems(n);
   if (kv == 4 || kv == 8 || kv == 16) E = kv;

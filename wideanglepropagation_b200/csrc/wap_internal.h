@@ -44,6 +44,8 @@ struct wap_plan {
   int row_e = 16, col_e = 16, col_w = 16;   // FFT launch shape (autotuned)
   float4* tw_row = nullptr;                 // twiddles for nx / row_e (hi, lo)
   float4* tw_col = nullptr;                 // twiddles for ny / col_e (hi, lo)
+  float4* tw_row8 = nullptr;                // the same for 8 elements per thread (medium passes),
+  float4* tw_col8 = nullptr;                // where row_e / col_e are 16 and the side allows it
   // WPM workspace
   float2* fields = nullptr;                 // (max_batch, n_bins, ny, nx)
   float2* dpbuf = nullptr;                  // (max_batch, ny, nx)
@@ -63,7 +65,7 @@ struct wap_plan {
   size_t ttab_cap = 0;
   wap::Detector det;                        // diffraction-pattern window (wap_plan_set_detector)
   unsigned long long* counter = nullptr;    // probe builder: aperture pixel count (allocated on first use)
-  // a grid with an axis that is not a power of two: Bluestein transforms
+  // a grid with an axis that is not a power of two: mixed-radix or Bluestein transforms
   bool generic = false;
   wap::GenAxis gen_x, gen_y;                // along x (rows) and y (columns)
   // one-launch chain of a single probe (wap_chain.cu): its twiddle table,
