@@ -544,9 +544,12 @@ def profile_cluster():
 
 def profile_chain():
     """C1 (Fresnel 256^2, 20 slices, one probe) through simulate_fresnel_as,
-    two calls: the case of the one-launch cooperative chain kernel."""
+    two calls, on the one-launch cooperative chain kernel (by override: a launch
+    per pass is the default there)."""
     import torch
     import wideanglepropagation_b200 as wap
+    from wideanglepropagation_b200 import _lib
+    _lib.check(_lib.lib().wap_scan_debug_override(_lib.WAP_KNOB_CHAIN, 4))
     w = wap.synthetic.plain_fresnel(0)
     dev = torch.device("cuda", 0)
     V = torch.as_tensor(w.potential[0], device=dev)

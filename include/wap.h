@@ -42,8 +42,8 @@ const char* wap_last_error(void);
 
 /* Create a plan for ny x nx grids and up to max_batch probes per call.  Sides
  * that are powers of two in [32, 2048] take the fast kernels; a grid with
- * another side (any n in [17, 1024]) runs Bluestein transforms through the
- * same FFT core (wap_multislice_fwd and wap_wpm_fwd only; the checkpointed
+ * another side (any n in [17, 1024]) runs mixed-radix lines, or Bluestein
+ * transforms where a prime above 7 divides it (wap_multislice_fwd and wap_wpm_fwd only; the checkpointed
  * forward, the adjoint, wap_spectrum_propagate and wap_aperture_probe return
  * WAP_ERR_UNSUPPORTED for such plans).  op is WAP_OP_*; n_bins is the WPM bin count
  * (ignored for WAP_OP_FRESNEL_AS).  Allocates twiddle tables and, for WPM,
@@ -54,8 +54,9 @@ int wap_plan_create(wap_plan** plan, int ny, int nx, int max_batch, int op, int 
 /* Release a plan and everything it allocated. */
 int wap_plan_destroy(wap_plan* plan);
 
-/* Status of the plan's last one-launch chain (single-probe forwards run all
- * slices in one cooperative kernel whose grid-wide waits are bounded): a copy
+/* Status of the plan's last one-launch chain (single-probe forwards on
+ * 128 x 128 where the cluster kernel is not to be had run all slices in one
+ * cooperative kernel whose grid-wide waits are bounded): a copy
  * of the status word (0 or WAP_ERR_TIMEOUT) into host_status, pinned host
  * memory, enqueued on `stream`; valid once the stream reaches it.  No
  * counterpart in the reference. */
