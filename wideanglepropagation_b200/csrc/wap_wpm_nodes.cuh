@@ -128,7 +128,14 @@ struct GroupColExchange {
 // Groups per line (G of the kernels below) when few lines are in flight.
 __host__ __device__ constexpr int node_col_groups(int n) { return n >= 2048 ? 1 : 2; }
 __host__ __device__ constexpr int node_row_groups(int n) { return n >= 2048 ? 1 : n >= 1024 ? 2 : 4; }
-__host__ __device__ constexpr int node_col_threads(int n, int g) { return n >= 1024 ? 512 * g : 256 * g; }
+// Threads and resident blocks of the column pass.  At 1024 points 512 threads hold
+// four columns, twice per SM (one 1024^2 probe, 40 slices: 3.09 ms with one block of
+// 128 registers per thread, 3.02 with two of 64), or two columns in two groups (1024 x
+// 256: 1.27 ms as one block of 1024 threads, 0.92 now).
+__host__ __device__ constexpr int node_col_threads(int n, int g) {
+  return n >= 2048 ? 512 * g : n >= 1024 ? 512 : 256 * g;
+}
+__host__ __device__ constexpr int node_col_blocks(int n, int g) { return g > 1 || n >= 2048 ? 1 : n >= 1024 ? 2 : 3; }
 
 // Column pass: column FFT, * Hvac * exp(i g(a0; q)), then per field its factor
 // and the inverse column FFT.  With G groups of threads per column tile, group 0
@@ -144,7 +151,7 @@ __host__ __device__ constexpr int node_col_threads(int n, int g) { return n >= 1
 // results, row by row.  Drift of |psi| over 200 slices of 512^2, rms over
 // specimens: 5.9e-7 without, 4.1e-8 with (the exit wave's error 2.0e-6, 1.5e-6).
 template <int NY, int E, int G>
-__global__ void __launch_bounds__(node_col_threads(NY, G), G == 1 && NY < 1024 ? 3 : 1)
+__global__ void __launch_bounds__(node_col_threads(NY, G), node_col_blocks(NY, G))
 wpm_node_col_kernel(const WpmNodeColArgs na) {
   using P = FFTPlan<NY, E>;
   constexpr int T = P::T;
