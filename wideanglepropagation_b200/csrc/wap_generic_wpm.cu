@@ -23,10 +23,11 @@ struct GenWpmSpectrum {       // column DFT -> spectrum * Hvac (* the centre nod
   const float2* hvac_lo;
   float2* spec;               // this column's spectrum, stride w
   float* dp;
+  float2 ref;                 // taken off the column k_x = 0 (0 elsewhere)
   float kx2, a0;
   int drx, w;
   bool nodes;
-  __device__ __forceinline__ float2 load(int p) const { return __ldcg(pcol + p * na.c.nx); }
+  __device__ __forceinline__ float2 load(int p) const { return csub(__ldcg(pcol + p * na.c.nx), ref); }
   __device__ __forceinline__ float2 turn(int, float2 y) const { return y; }
   __device__ __forceinline__ void store(int p, float2 y) const {
     if (dp) {
@@ -51,6 +52,7 @@ struct GenWpmField {          // spectrum * the field's factor -> inverse column
   const float2* hvac;
   const float2* spec;
   float2* fcol;
+  float2 ch, cl;              // the part taken off, propagated: added to every row
   float kx2, a0, da;          // da: a_k of a reference field
   int w, k;
   bool nodes;
@@ -74,7 +76,9 @@ struct GenWpmField {          // spectrum * the field's factor -> inverse column
     return cconj(u);
   }
   __device__ __forceinline__ float2 turn(int, float2 y) const { return y; }
-  __device__ __forceinline__ void store(int p, float2 y) const { __stcg(fcol + p * na.c.nx, cconj(y)); }
+  __device__ __forceinline__ void store(int p, float2 y) const {
+    __stcg(fcol + p * na.c.nx, cadd(cadd(cconj(y), cl), ch));
+  }
 };
 
 // Block group z forms the fields z, z + gridDim.z, ... (each repeats the forward
@@ -115,6 +119,10 @@ __global__ void __launch_bounds__(BLUE ? kGenThreads : 2 * kGenThreads, BLUE ? 3
   __syncthreads();
   pdl_wait_then_release();
   if (!a.dp_mode && (int)blockIdx.z >= nf) return;
+  // the column k_x = 0 less its first element, whose share is propagated beside it
+  // (wpm_node_col_kernel)
+  const bool apart = nodes && !a.dp_mode && live && col == 0;
+  fwd.ref = apart ? __ldcg(a.psi + (long long)b * plane) : make_float2(0.f, 0.f);
   mix_pass<BLUE>(ax, 1, tw, mem, t, live, fwd);
   if (a.dp_mode) return;
   GenWpmField inv{na};
@@ -124,11 +132,29 @@ __global__ void __launch_bounds__(BLUE ? kGenThreads : 2 * kGenThreads, BLUE ? 3
   inv.a0 = fwd.a0;
   inv.w = w;
   inv.nodes = nodes;
+  float2 ch = make_float2(0.f, 0.f), cl = ch;
+  float rest0 = 0.f;
+  if (apart) {
+    const float k2 = __ldg(a.ky2) + fwd.kx2, a0 = fwd.a0;
+    rest0 = wpm_slope_rest(a.k02 + a0 - k2, (na.dq - a0 + k2) * na.inv_qbar, na.kappa, na.inv_root_qbar);
+    const float2 m = cism1(a0 * wpm_mean_slope(rest0, na.kappa, -a0, a.dz, na.c4));
+    const float2 h = __ldg(fwd.hvac), l = __ldg(fwd.hvac_lo), r = fwd.ref;
+    const double hx = (double)h.x + (h.x * m.x - h.y * m.y + l.x), hy = (double)h.y + (h.x * m.y + h.y * m.x + l.y);
+    const double cx = a.ny * (r.x * hx - r.y * hy), cy = a.ny * (r.x * hy + r.y * hx);
+    ch = make_float2((float)cx, (float)cy);
+    cl = make_float2((float)(cx - ch.x), (float)(cy - ch.y));
+  }
   for (int k = blockIdx.z; k < nf; k += gridDim.z) {
     __syncthreads();   // the spectrum is complete, and the last pass's buffers are free
     inv.k = k;
+    inv.ch = ch;
+    inv.cl = cl;
     if (nodes) {
       inv.da = rec->da[k];
+      if (apart && k > 0) {
+        inv.ch = cmul(ch, cism1(inv.da * wpm_mean_slope(rest0, na.kappa, inv.da, a.dz, na.c4)));
+        inv.cl = make_float2(0.f, 0.f);
+      }
     } else {
       const float dk = a.refs[srow * a.K + k];
       inv.da = a.k02 * dk * (2.0f + dk);   // n_k^2 k0^2 - k0^2
