@@ -64,10 +64,12 @@ __global__ void __launch_bounds__(kRowThreads) blue_row_kernel(const GenRowArgs 
   const int rl = threadIdx.x / T, t = threadIdx.x - rl * T;
   const int row = blockIdx.x * a.rows + rl;
   const bool live = row < a.ny;
+  const bool first = a.flags & ROW_LOAD_SRC;
+  if (first) pdl_wait_then_release();
   GenRowOp op = gen_row_op(a, a.probe0 + blockIdx.y, live ? row : 0);
   const RowExchange<(T <= 32)> xs{xbuf + rl * PADN};
   __syncthreads();
-  pdl_wait_then_release();
+  if (!first) pdl_wait_then_release();
   blue_pass<M, E>(a.ax, (a.flags & (ROW_IFFT | ROW_FFT)) == (ROW_IFFT | ROW_FFT) ? 2 : 1, tw, xs, t, live, op);
 }
 

@@ -34,6 +34,8 @@ __global__ void __launch_bounds__(BLUE ? kGenThreads : 2 * kGenThreads, BLUE ? 3
   const int row = blockIdx.x * rows + rl;
   const bool live = rl < rows && row < a.ny;
   const int b = a.probe0 + blockIdx.y;
+  const bool first = a.flags & ROW_LOAD_SRC;
+  if (first) pdl_wait_then_release();
   GenRowOp op = gen_row_op(a, b, row);
   const MixMem mem{bufs + min(rl, rows - 1) * ax.m, rows * ax.m, 1};
   if (a.fetch) {
@@ -45,7 +47,7 @@ __global__ void __launch_bounds__(BLUE ? kGenThreads : 2 * kGenThreads, BLUE ? 3
     op.trow = ts + rl * a.nx;
   }
   __syncthreads();
-  pdl_wait_then_release();
+  if (!first) pdl_wait_then_release();
   mix_pass<BLUE>(ax, (a.flags & (ROW_IFFT | ROW_FFT)) == (ROW_IFFT | ROW_FFT) ? 2 : 1, tw, mem, t, live, op);
 }
 

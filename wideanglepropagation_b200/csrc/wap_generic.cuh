@@ -92,6 +92,10 @@ struct GenRowOp {
   }
 };
 
+// Reads the call's positions and draw indices.  The kernel before the first pass of a
+// call (ROW_LOAD_SRC) may be the one that writes them, and its writes are visible only
+// after the dependent-launch wait, so that pass waits before it comes here; later
+// passes come here ahead of their wait, two launches after whatever wrote them.
 __device__ __forceinline__ GenRowOp gen_row_op(const GenRowArgs& a, int b, int row) {
   GenRowOp op{a};
   op.f = a.flags;

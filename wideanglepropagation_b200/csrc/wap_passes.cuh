@@ -161,16 +161,19 @@ static __global__ void __launch_bounds__(256) interleave_h_kernel(const float2* 
 // with the attribute may become resident while the previous kernel in the
 // stream drains; griddepcontrol.wait then blocks until that kernel has
 // completed and its writes are visible (a no-op for a normal launch), and
-// launch_dependents lets the next pass start the same way.  Both come first
-// in the kernel, before any global read.
+// launch_dependents lets the next pass start the same way.  Ahead of the two a
+// kernel may read only what no kernel launched directly before it can have
+// written: a plan's constant tables, and from a call's second pass on the
+// call's own inputs and whatever was complete before its first pass (that pass
+// has waited for it).  All other reads, and every write, come after the wait.
 __device__ __forceinline__ void pdl_wait_then_release() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Row and column passes go out with programmatic dependent launch (the
-// kernels wait for their predecessor first thing): in a chain of short,
-// latency-bound passes the next pass is already resident when one finishes
+// Row and column passes go out with programmatic dependent launch (see
+// pdl_wait_then_release for what they may read before their wait): in a chain of
+// short, latency-bound passes the next pass is already resident when one finishes
 // (C1 0.26 -> 0.19 ms per call).  The reference-field WPM passes launch normally:
 // their large CTAs parked early cost more than the launch latency saved (C3 12.5 vs 13.1 ms).
 template <class K, class A>
