@@ -66,3 +66,59 @@ def test_positions_written_just_before_the_call(wap, ny, nx):
         got = [o.clone() for o in out]
         for a, b in zip(got, call(s)):
             assert _close(a, b)
+
+
+def test_general_grid_goes_without_the_plans_table(wap):
+    """A captured call on a grid that is not a power of two reads no memory of
+    the plan that another call writes: no table kernel (2 N + 1 passes)."""
+    from wideanglepropagation_b200 import _lib
+    V, probe, H, dz, E = _case(wap, 48, 60, 3)
+
+    def call():
+        return wap.simulate_fresnel_as(V, probe, H, dz, E, return_wavefronts=False)[:2]
+
+    want = call()
+    n0 = _lib.launch_count()
+    g, out = _captured(call)
+    assert _lib.launch_count() - n0 == 2 * 3 + 1
+    g.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(out, want):
+        assert _close(a, b)
+
+
+def _wpm(wap, V, probe, dz, E, **kw):
+    return wap.simulate_wpm(V, probe, dz, E, (0.1, 0.1), 6, 1.0, return_wavefronts=False, **kw)[:2]
+
+
+@pytest.mark.parametrize("kind", ["scan", "wpm"])
+def test_larger_calls_leave_a_captured_one_valid(wap, kind):
+    """Later calls on the cached plan with more slices (its table and records are
+    replaced by larger ones) and with more probes (the plan is)."""
+    n, B = (128, 16) if kind == "scan" else (64, 3)
+    V, probe, H, dz, E = _case(wap, n, n, 12)
+    pos = torch.from_numpy(np.random.default_rng(2).integers(0, n, (B, 2)).astype(np.int32)).cuda()
+    many = pos.repeat(5, 1)
+
+    def call(k, p=pos):
+        if kind == "wpm":
+            return _wpm(wap, V[:k], probe, dz, E, positions=p)
+        return wap.simulate_fresnel_as(V[:k], probe, H, dz, E, positions=p, return_wavefronts=False)[:2]
+
+    want = [o.clone() for o in call(3)]
+    g, out = _captured(lambda: call(3))
+    call(12)
+    if kind == "wpm":
+        _wpm(wap, V, probe, dz, E, positions=many)
+    else:   # 80 different waves: past the cached plan's 64
+        wap.simulate_fresnel_as(V, probe.repeat(80, 1, 1), H, dz, E, return_wavefronts=False)
+    fill = [torch.full((1 << 20,), float("nan"), device="cuda") for _ in range(8)]
+    for o in out:
+        o.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    del fill
+    for a, b in zip(out, want):
+        assert _close(a, b)
+    del g
+    wap.release_caches()

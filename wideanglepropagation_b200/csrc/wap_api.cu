@@ -342,6 +342,7 @@ static void plan_free(wap_plan* p) {
   cudaFree(p->wn_tw_row);
   cudaFree(p->wn_tw_col);
   cudaFree(p->ttab);
+  for (void* d : p->kept) cudaFree(d);
   cudaFree(p->counter);
   cudaFree(p->chain_tw);
   cudaFree(p->chain_count);
@@ -612,16 +613,34 @@ static bool use_trans_table(const wap_plan* p, int n_probes, int n_slices, int n
   return (size_t)n_draws * n_slices * p->ny * p->nx * sizeof(float2) <= kSmallTransTable;
 }
 
-// exp(i phi(V)) for every draw and slice into the plan's grow-only table
+int stream_capture(cudaStream_t st) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
+  }
+  return status != cudaStreamCaptureStatusNone;
+}
+
+void drop_outgrown(wap_plan* p, void* d, bool captured) {
+  if (d && captured) p->kept.push_back(d);
+  else cudaFree(d);
+}
+
+// exp(i phi(V)) for every draw and slice into the plan's grow-only table.  A graph
+// holds the table's address for as long as it is replayed, so a table that a captured
+// call has used is kept when it grows.  Captured calls on grids that are not powers
+// of two hold no memory of the plan that other calls write, and go without.
 int build_trans_table(wap_plan* p, const float* V, int n_slices, int n_draws, const RowArgs& r, cudaStream_t st) {
   const size_t need = (size_t)n_draws * n_slices * p->ny * p->nx;
   cudaError_t e = cudaSuccess;
+  const int capture = stream_capture(st);
+  // a stream in capture may not allocate: the passes evaluate exp(i phi) inline
+  if ((capture == 1 && p->generic) || (capture && need > p->ttab_cap))
+    return fail(WAP_ERR_CUDA, "transmission table: the stream is being captured");
   if (need > p->ttab_cap) {
-    // a stream in capture may not allocate: the passes evaluate exp(i phi) inline
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)
-      return fail(WAP_ERR_CUDA, "transmission table: the stream is being captured");
-    cudaFree(p->ttab);
+    drop_outgrown(p, p->ttab, p->ttab_captured);
+    p->ttab_captured = false;
     p->ttab = nullptr;
     p->ttab_cap = 0;
     e = cudaMalloc(&p->ttab, need * sizeof(float2));
@@ -631,6 +650,7 @@ int build_trans_table(wap_plan* p, const float* V, int n_slices, int n_draws, co
     }
     p->ttab_cap = need;
   }
+  if (capture == 1) p->ttab_captured = true;
   const long long n4 = (long long)need / 4;
   const ProfToken tok = prof_begin(WAP_KIND_TRANS, st);
   count_launch();

@@ -63,6 +63,9 @@ struct wap_plan {
   float4* wn_tw_col = nullptr;
   float2* ttab = nullptr;                   // transmission table (draws, n_slices, ny, nx)
   size_t ttab_cap = 0;
+  // buffers that a captured call reads: kept when larger ones take their places, until the plan goes
+  bool ttab_captured = false, refs_captured = false;
+  std::vector<void*> kept;
   wap::Detector det;                        // diffraction-pattern window (wap_plan_set_detector)
   unsigned long long* counter = nullptr;    // probe builder: aperture pixel count (allocated on first use)
   // a grid with an axis that is not a power of two: mixed-radix or Bluestein transforms
@@ -98,6 +101,11 @@ const char* last_error();
 
 int check_common(const wap_plan* p, const float* V, int n_slices, int n_draws, const float* psi0, int n_probes,
                  float* exit);
+// whether a stream is being captured: 1, 0, or -1 where the runtime will not say
+int stream_capture(cudaStream_t st);
+// gives up a buffer that a plan has outgrown: freed, or kept with the plan where a
+// captured call holds its address
+void drop_outgrown(wap_plan* p, void* d, bool captured);
 int rows_per_cta(int nx, int e, int ny, int nb);
 bool size_supported(int n);
 

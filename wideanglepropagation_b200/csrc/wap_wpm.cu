@@ -344,20 +344,22 @@ static int wpm_slices(wap_plan* p, const float* V, int n_slices, int n_draws, co
   const size_t rows = (size_t)n_draws * n_slices;
   cudaError_t e;
   if (rows * K > p->refs_cap) {
-    cudaFree(p->refs);
+    drop_outgrown(p, p->refs, p->refs_captured);
     p->refs = nullptr;
     p->refs_cap = 0;
     if ((e = cudaMalloc(&p->refs, rows * K * sizeof(float))) != cudaSuccess) return cuda_fail(e, "cudaMalloc(refs)");
     p->refs_cap = rows * K;
   }
-  if (rows > p->slices_cap) {
-    cudaFree(p->slices);
+  if (rows > p->slices_cap) {   // (grows with refs: K is the plan's)
+    drop_outgrown(p, p->slices, p->refs_captured);
+    p->refs_captured = false;
     p->slices = nullptr;
     p->slices_cap = 0;
     if ((e = cudaMalloc(&p->slices, rows * sizeof(WpmSlice))) != cudaSuccess)
       return cuda_fail(e, "cudaMalloc(WPM records)");
     p->slices_cap = rows;
   }
+  if (stream_capture(st) == 1) p->refs_captured = true;
   const double qmin = ph.k0 * ph.k0 - (k2_max(p->ny, sampling_y) + k2_max(p->nx, sampling_x));
   out->nodes = qmin > 0.0 && std::fabs(dz) >= 1e-6;
   if (out->nodes) {

@@ -214,7 +214,8 @@ class StreamOrder:
 
 class Plan:
     """Owns one ``wap_plan`` (twiddle tables, WPM workspace) on one device;
-    ``order`` keeps its uses from different streams apart."""
+    ``order`` keeps its uses from different streams apart.  ``captured``: a call
+    in a CUDA graph capture has used it, so a graph may hold its addresses."""
 
     def __init__(self, ny: int, nx: int, max_batch: int, op: int, n_bins: int = 0):
         L = _lib.lib()
@@ -225,9 +226,12 @@ class Plan:
         self.device = torch.cuda.current_device()
         self.det = None
         self.order = StreamOrder()
+        self.captured = False
 
     def begin(self):
         """The current stream, after the plan's last use on another stream."""
+        if torch.cuda.is_current_stream_capturing():
+            self.captured = True
         return self.order.begin(torch.cuda.current_stream(self.device))
 
     def end(self, cur) -> None:
@@ -265,6 +269,7 @@ class Plan:
 
 
 _plans: dict = {}
+_outgrown: list = []   # captured plans that a larger one has replaced: kept until release_caches
 _plans_lock = threading.Lock()
 
 
@@ -279,7 +284,9 @@ def get_plan(ny: int, nx: int, batch: int, op: int, n_bins: int = 0) -> Plan:
     with _plans_lock:
         p = _plans.get(key)
         if p is None or p.max_batch < batch:
-            if p is not None:
+            if p is not None and p.captured:
+                _outgrown.append(p)
+            elif p is not None:
                 p.close()
             cap = batch if (op == _lib.WAP_OP_WPM or cls == "single") else max(batch, 64)
             p = Plan(ny, nx, cap, op, n_bins)
@@ -591,9 +598,10 @@ def release_caches() -> None:
             _lib.lib().wap_scan_destroy(h)
         _scans.clear()
     with _plans_lock:
-        for p in _plans.values():
+        for p in [*_plans.values(), *_outgrown]:
             p.close()
         _plans.clear()
+        _outgrown.clear()
     from . import autograd
     autograd.release_pool()
 
