@@ -208,7 +208,8 @@ struct RowCfg {
 template <int E>
 __host__ __device__ constexpr int early_elems() { return E <= 8 ? E : 1; }
 
-// this thread's elements of the transmission row, read through L2
+// this thread's elements of the transmission row, through L1: the probes of a draw
+// read the same rows (4096 probes of 32^2, 20 slices: 0.79 ms, 1.05 through L2 alone)
 template <int NX, int E>
 __device__ __forceinline__ void row_fetch_t(const RowArgs& a, int bx, int by, float2 (&tpre)[early_elems<E>()]) {
   constexpr int T = RowCfg<NX, E>::T;
@@ -217,7 +218,7 @@ __device__ __forceinline__ void row_fetch_t(const RowArgs& a, int bx, int by, fl
   const int d = a.draw ? a.draw[b] : 0;
   const float2* trow = a.ttab + (long long)d * a.v_draw_stride + ((long long)a.slice * a.ny + row) * NX;
 #pragma unroll
-  for (int e = 0; e < early_elems<E>(); ++e) tpre[e] = __ldcg(trow + t + T * e);
+  for (int e = 0; e < early_elems<E>(); ++e) tpre[e] = __ldg(trow + t + T * e);
 }
 
 // One row tile (rows blockDim.x / T consecutive rows of probe probe0 + by):
