@@ -68,10 +68,16 @@ int wap_plan_status_async(wap_plan* plan, int* host_status, void* stream);
 int wap_plan_status_pending(wap_plan* plan, int* pending);
 
 /* FFT launch shape of the row pass (elements per thread) and column pass
- * (elements per thread, columns per CTA); set by the autotuner.  Elements
- * per thread: 8 or 16, and 4 for Fresnel/AS plans on grids up to 1024;
- * WAP_ERR_ARG for a shape the kernels cannot launch. */
+ * (elements per thread, columns per CTA).  Elements per thread: 8 or 16, and 4
+ * for Fresnel/AS plans on grids up to 1024; WAP_ERR_ARG for a shape the kernels
+ * cannot launch.  wap_plan_set_config: every later pass has exactly this shape
+ * (WPM plans: the first row pass, the pattern, and the slices of grids that
+ * reach the evanescent edge; the interpolating passes of the others have shapes
+ * of their own).  wap_plan_hint_config: the shape is one found on batches that
+ * fill the chip, and passes of fewer pixels may take shorter lines per thread
+ * and fewer columns (the default of a plan; the autotuner's cached shapes). */
 int wap_plan_set_config(wap_plan* plan, int row_e, int col_e, int col_w);
+int wap_plan_hint_config(wap_plan* plan, int row_e, int col_e, int col_w);
 int wap_plan_get_config(const wap_plan* plan, int* row_e, int* col_e, int* col_w);
 
 /* Detector window of the diffraction pattern for the plan's later calls:

@@ -40,6 +40,7 @@ SIGNATURES = {
     "wap_plan_create": (_I, [ctypes.POINTER(_P), _I, _I, _I, _I, _I]),
     "wap_plan_destroy": (_I, [_P]),
     "wap_plan_set_config": (_I, [_P, _I, _I, _I]),
+    "wap_plan_hint_config": (_I, [_P, _I, _I, _I]),
     "wap_plan_set_detector": (_I, [_P, _I, _I, _I, _I]),
     "wap_gaussian_potential": (_I, [_I, _I, _I, _D, _D, _P, _P, _D, _D, _P, _P]),
     "wap_aperture_probe": (_I, [_P, _D, _D, _D, _D, _D, _I, _P, _P]),

@@ -136,7 +136,7 @@ def tune(ny: int, nx: int, op: int = 0, n_bins: int = 0, batch: int | None = Non
         if verbose:
             print(f"  {ny}x{nx} op{op} {cfg}: {times[cfg]:.3f} ms", flush=True)
     best = min(times, key=times.get)
-    plan.set_config(*best) if best else plan.set_config(*old)
+    plan.hint_config(*(best or old))
     store(ny, nx, op, n_bins, best, batch_class(batch))
     return best, times
 

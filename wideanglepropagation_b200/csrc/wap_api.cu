@@ -290,7 +290,7 @@ static int upload_twiddles(wap_plan* p) {
     if (d) cudaFree(d);
     d = nullptr;
     if (which >= 2) {
-      if (e != 16 || n < 128 || n > 1024) continue;
+      if (p->exact_shape || e != 16 || n < 128 || n > 1024) continue;
       e = 8;
     }
     std::vector<float4> h = twiddle_table(n, e);
@@ -427,8 +427,7 @@ int wap_plan_destroy(wap_plan* p) {
   return WAP_OK;
 }
 
-int wap_plan_set_config(wap_plan* p, int row_e, int col_e, int col_w) {
-  clear_error();
+static int plan_shape(wap_plan* p, int row_e, int col_e, int col_w, bool exact) {
   if (!p) return fail(WAP_ERR_ARG, "plan is NULL");
   if (p->generic) return fail(WAP_ERR_UNSUPPORTED, "grids that are not powers of two have a fixed launch shape");
   if (!config_valid(p, row_e, col_e, col_w))
@@ -437,7 +436,18 @@ int wap_plan_set_config(wap_plan* p, int row_e, int col_e, int col_w) {
   p->row_e = row_e;
   p->col_e = col_e;
   p->col_w = col_w;
+  p->exact_shape = exact;
   return upload_twiddles(p);
+}
+
+int wap_plan_set_config(wap_plan* p, int row_e, int col_e, int col_w) {
+  clear_error();
+  return plan_shape(p, row_e, col_e, col_w, true);
+}
+
+int wap_plan_hint_config(wap_plan* p, int row_e, int col_e, int col_w) {
+  clear_error();
+  return plan_shape(p, row_e, col_e, col_w, false);
 }
 
 int wap_plan_set_detector(wap_plan* p, int y0, int x0, int ny, int nx) {
@@ -554,7 +564,7 @@ static double col_bytes(const wap_plan* p, const ColArgs& c, int n_probes) {
 // batch chunks of at most 65535 probes (grid.y limit)
 // A shape of 16 elements per thread was chosen for a full chip.  Passes of at most
 // kMediumRows pixels take 8 along the rows, of at most kMediumCols along the columns:
-// more and shorter threads.  Measured per slice (row e, column e, columns per CTA):
+// more and shorter threads (tw_row8, tw_col8: plans whose shape the caller has not set).  Measured per slice (row e, column e, columns per CTA):
 // 16 probes on 256^2 15.5 -> 14.7 us, 4 on 512^2 20.6 -> 19.0, 8 on 256^2 11.6 -> 10.5
 // with 8 columns; 4 on 256^2 9.2 -> 8.1, 16 on 128^2 8.6 -> 7.0 with short columns too;
 // from 3 probes on 1024^2 on, 16 stays the faster (62.5 against 65.8).
@@ -590,7 +600,7 @@ cudaError_t col_chunks(const wap_plan* p, ColArgs c, int n_probes, cudaStream_t 
     }
   }
   const int T = p->ny / elems;
-  while (w > 4 && w * T > 64 && (long long)(p->nx / w) * n_probes < kFewCtas) w >>= 1;
+  while (!p->exact_shape && w > 4 && w * T > 64 && (long long)(p->nx / w) * n_probes < kFewCtas) w >>= 1;
   const ProfToken tok = prof_begin(WAP_KIND_COL, st);
   for (int b0 = 0; b0 < n_probes; b0 += 65535) {
     c.probe0 = b0;

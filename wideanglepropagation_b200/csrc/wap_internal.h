@@ -42,6 +42,7 @@ struct wap_plan {
   int device = 0;
   int ny = 0, nx = 0, max_batch = 0, op = 0, n_bins = 0;
   int row_e = 16, col_e = 16, col_w = 16;   // FFT launch shape (autotuned)
+  bool exact_shape = false;                 // set by the caller: launched as it is (else row_chunks, col_chunks)
   float4* tw_row = nullptr;                 // twiddles for nx / row_e (hi, lo)
   float4* tw_col = nullptr;                 // twiddles for ny / col_e (hi, lo)
   float4* tw_row8 = nullptr;                // the same for 8 elements per thread (medium passes),

@@ -238,7 +238,12 @@ class Plan:
         self.order.end(cur)
 
     def set_config(self, row_e: int, col_e: int, col_w: int) -> None:
+        """Launch every later pass in exactly this shape."""
         _lib.check(_lib.lib().wap_plan_set_config(self.handle, row_e, col_e, col_w))
+
+    def hint_config(self, row_e: int, col_e: int, col_w: int) -> None:
+        """The shape of batches that fill the chip; smaller passes may take shorter ones."""
+        _lib.check(_lib.lib().wap_plan_hint_config(self.handle, row_e, col_e, col_w))
 
     def set_detector(self, det) -> None:
         """Diffraction-pattern window (y0, x0, ny, nx) of later calls; None: whole grid."""
@@ -292,7 +297,7 @@ def get_plan(ny: int, nx: int, batch: int, op: int, n_bins: int = 0) -> Plan:
             p = Plan(ny, nx, cap, op, n_bins)
             cfg = autotune.lookup(ny, nx, op, n_bins, cls)
             if cfg is not None:
-                p.set_config(*cfg)
+                p.hint_config(*cfg)
             _plans[key] = p
         p.set_detector(None)   # cached plans are shared: whole-grid patterns unless a caller sets a window
         return p
