@@ -393,8 +393,8 @@ int wap_plan_create(wap_plan** out, int ny, int nx, int max_batch, int op, int n
   p->col_e = elems(ny, true);
   p->col_w = default_col_w(ny, p->col_e, nx);
   p->generic = generic;
-  int rc = generic ? generic_axis_create(&p->gen_x, nx, op == WAP_OP_WPM) : upload_twiddles(p);
-  if (rc == WAP_OK && generic) rc = generic_axis_create(&p->gen_y, ny, op == WAP_OP_WPM);
+  int rc = generic ? generic_axis_create(&p->gen_x, nx) : upload_twiddles(p);
+  if (rc == WAP_OK && generic) rc = generic_axis_create(&p->gen_y, ny);
   if (rc != WAP_OK) {
     plan_free(p);   // keeps the failure's message
     return rc;

@@ -22,8 +22,7 @@
 
 namespace wap {
 
-template <bool BLUE>
-__global__ void __launch_bounds__(BLUE ? kGenThreads : 2 * kGenThreads, BLUE ? 3 : 2) gen_row_kernel(const GenRowArgs a) {
+__global__ void __launch_bounds__(2 * kGenThreads, 2) gen_row_kernel(const GenRowArgs a) {
   extern __shared__ float4 gen_smem[];
   const GenAxis& ax = a.ax;
   const int T = ax.threads, rows = a.rows;
@@ -48,7 +47,7 @@ __global__ void __launch_bounds__(BLUE ? kGenThreads : 2 * kGenThreads, BLUE ? 3
   }
   __syncthreads();
   if (!first) pdl_wait_then_release();
-  mix_pass<BLUE>(ax, (a.flags & (ROW_IFFT | ROW_FFT)) == (ROW_IFFT | ROW_FFT) ? 2 : 1, tw, mem, t, live, op);
+  mix_pass(ax, (a.flags & (ROW_IFFT | ROW_FFT)) == (ROW_IFFT | ROW_FFT) ? 2 : 1, tw, mem, t, live, op);
 }
 
 __global__ void __launch_bounds__(2 * kGenThreads, 2) gen_col_kernel(const GenColArgs a) {
@@ -78,7 +77,7 @@ __global__ void __launch_bounds__(2 * kGenThreads, 2) gen_col_kernel(const GenCo
   }
   __syncthreads();
   pdl_wait_then_release();
-  mix_pass<false>(ax, 2, tw, mem, t, live, op);
+  mix_pass(ax, 2, tw, mem, t, live, op);
 }
 
 // exp(i phi(V)) of every slice, any pixel count
@@ -92,17 +91,16 @@ __global__ void __launch_bounds__(256) gen_trans_table_kernel(const float* __res
 // launches
 // ----------------------------------------------------------------------------
 cudaError_t launch_gen_row(GenRowArgs& a, int nb, cudaStream_t st) {
-  if (a.ax.pow2) return launch_blue_row(a, nb, st);
+  if (a.ax.blue) return launch_blue_row(a, nb, st);
   a.rows = gen_lines(a.ny, a.ax.threads, 64, std::max(1, 32 / a.ax.threads), kGenThreads, nb);
   a.fetch = a.tab_ready && (a.flags & ROW_TRANS_TAB) && gen_fetch(a.ax, (long long)a.ny * nb);
   const size_t smem =
       a.ax.tw_len * sizeof(float4) + (size_t)a.rows * (2 * a.ax.m + (a.fetch ? a.nx : 0)) * sizeof(float2);
-  return launch_gen(a.ax.blue ? gen_row_kernel<true> : gen_row_kernel<false>, dim3((a.ny + a.rows - 1) / a.rows, nb),
-                    a.rows * a.ax.threads, smem, st, a);
+  return launch_gen(gen_row_kernel, dim3((a.ny + a.rows - 1) / a.rows, nb), a.rows * a.ax.threads, smem, st, a);
 }
 
 static cudaError_t launch_gen_col(GenColArgs& a, int nb, cudaStream_t st) {
-  if (a.ax.pow2) return launch_blue_col(a, nb, st);
+  if (a.ax.blue) return launch_blue_col(a, nb, st);
   a.w = gen_cols(a.ax, a.nx, nb);
   a.fetch = gen_fetch(a.ax, (long long)a.nx * nb);
   const size_t smem = a.ax.tw_len * sizeof(float4) +
@@ -202,7 +200,6 @@ static int smooth_axis_tables(GenAxis* ax, const std::vector<int>& radices) {
   ax->stages = (int)radices.size();
   for (int s = 0; s < ax->stages; ++s) ax->radix[s] = radices[s];
   ax->threads = ax->m / *std::min_element(radices.begin(), radices.end());
-  if (ax->blue) ax->threads = std::min(ax->threads, kGenThreads);
   std::vector<float4> tw;
   stage_twiddles(radices, &tw);
   const std::vector<int> rev(radices.rbegin(), radices.rend());
@@ -214,44 +211,22 @@ static int smooth_axis_tables(GenAxis* ax, const std::vector<int>& radices) {
   return upload_vec(&ax->tw, tw);
 }
 
-int generic_axis_create(GenAxis* ax, int n, bool wpm) {
+int generic_axis_create(GenAxis* ax, int n) {
   *ax = GenAxis{};
   ax->n = ax->m = n;
   std::vector<int> radices;
-  if (!plan_radices(n, &radices)) {
-    ax->blue = 1;
-    if (wpm) {
-      // the smooth length from 2 n - 1 on with the fewest points x stages (2048 = 8 8 8 4 at the latest)
-      long long best = -1;
-      for (int m = 2 * n - 1; m <= 2048; ++m) {
-        std::vector<int> r;
-        if (!plan_radices(m, &r)) continue;
-        const long long cost = (long long)m * r.size();
-        if (best < 0 || cost < best) {
-          best = cost;
-          ax->m = m;
-          radices = r;
-        }
-      }
-    } else {
-      // power-of-two lines in registers (wap_bluestein.cu)
-      ax->pow2 = 1;
-      ax->m = 64;
-      while (ax->m < 2 * n - 1) ax->m <<= 1;
-    }
-  }
-  int rc;
-  if (ax->pow2) {
-    std::vector<float4> tw = twiddle_table(ax->m, 8);
-    ax->tw_rev = (int)tw.size();
-    const std::vector<float4> tw16 = twiddle_table(ax->m, 16);
-    tw.insert(tw.end(), tw16.begin(), tw16.end());
-    ax->tw_len = (int)tw.size();
-    if ((rc = upload_vec(&ax->tw, tw))) return rc;
-  } else {
-    if ((rc = smooth_axis_tables(ax, radices))) return rc;
-  }
-  if (!ax->blue) return rc;
+  if (plan_radices(n, &radices)) return smooth_axis_tables(ax, radices);
+  // Bluestein through power-of-two lines in registers (wap_bluestein.cu)
+  ax->blue = 1;
+  ax->m = 64;
+  while (ax->m < 2 * n - 1) ax->m <<= 1;
+  std::vector<float4> tw = twiddle_table(ax->m, 8);
+  ax->tw_rev = (int)tw.size();
+  const std::vector<float4> tw16 = twiddle_table(ax->m, 16);
+  tw.insert(tw.end(), tw16.begin(), tw16.end());
+  ax->tw_len = (int)tw.size();
+  int rc = upload_vec(&ax->tw, tw);
+  if (rc) return rc;
   // chirp w_q = exp(-i pi q^2 / n) with q^2 reduced mod 2n (exact integers)
   const int m = ax->m;
   std::vector<float4> chirp(n);

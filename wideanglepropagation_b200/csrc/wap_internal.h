@@ -21,18 +21,17 @@ struct Detector {
 
 struct WpmSlice;   // a slice's WPM record (wap_wpm_nodes.cuh)
 
-// One axis of a grid that is not a power of two (wap_mixed.cuh): a length-n DFT
-// by stages of radices 2 .. 8, or as Bluestein's chirp convolution through such
-// transforms of a length m >= 2n - 1.  Device pointers; tables of float64 values
-// stored as float hi + lo parts.
+// One axis of a grid that is not a power of two: a length-n DFT by stages of radices
+// 2 .. 8 (wap_mixed.cuh; m = n), or, with blue, as Bluestein's chirp convolution
+// through transforms of a power of two m >= 2n - 1 (wap_bluestein.cu).  Device
+// pointers; tables of float64 values stored as float hi + lo parts.
 struct GenAxis {
   int n = 0, m = 0, blue = 0, stages = 0;
-  int pow2 = 0;                     // Bluestein on the power-of-two core: tw holds the tables of 8 and
-                                    // (from tw_rev) 16 elements per thread; no stages
   int radix[5] = {0, 0, 0, 0, 0};
-  int threads = 0;                  // per line: m / smallest radix, at most 256
-  int tw_rev = 0, tw_len = 0;       // offset of the reversed order's twiddles, entries of both
+  int threads = 0;                  // per line: n / smallest radix
+  int tw_rev = 0, tw_len = 0;       // offset of the second table, entries of both
   const float4* tw = nullptr;       // stage twiddles, radices in order, then in reverse order
+                                    // (blue: the m-point tables of 8, then of 16 elements per thread)
   const float4* chirp = nullptr;    // (n) w_p = exp(-i pi p^2 / n)
   const float4* bhat = nullptr;     // (m) fft_m(b) / m, b_q = conj(w_q) on the circular index range
 };
@@ -144,7 +143,7 @@ int wpm_node_twiddles(wap_plan* p);
 
 // grids that are not powers of two (wap_generic.cu)
 bool generic_size_supported(int n);
-int generic_axis_create(GenAxis* ax, int n, bool wpm);
+int generic_axis_create(GenAxis* ax, int n);
 void generic_axis_free(GenAxis* ax);
 int generic_fresnel_forward(wap_plan* p, const RowArgs& r, const ColArgs& c, int n_slices, int n_probes,
                             float2* stack, cudaStream_t st);

@@ -1,22 +1,20 @@
 // Mixed-radix line transforms for grid sides that are not powers of two.
 //
 // A length-n DFT runs as up to five Stockham stages of radices 2 .. 8 (n a
-// product of such radices), or, where a prime above 7 divides n, as Bluestein's
-// chirp convolution through two such transforms of a smooth length m >= 2 n - 1.
+// product of such radices; sides with a prime above 7: wap_bluestein.cu).
 // The radices are run-time values (any side, one kernel); larger ones (up to 16)
 // halve the exchanges but not the time: their code, run once per block, and 200
 // registers per thread made a 240 x 300 x 16 pass 91 us.
-// A line belongs to T = m / (smallest radix) threads, one butterfly each per stage
-// (Bluestein's: at most 256 threads, every T-th butterfly); stages exchange through two shared-memory buffers in turn (one barrier
-// per stage).  A pass over a line is a chain of DFTs with a pointwise product
-// between them: the last stage of a transform and the first of the next have the
+// A line belongs to T = n / (smallest radix) threads, one butterfly each per stage;
+// stages exchange through two shared-memory buffers in turn (one barrier per stage).
+// A pass over a line is a chain of DFTs with a pointwise product between them: the last stage of a transform and the first of the next have the
 // same radix (every second transform takes the radices in reverse order), so the
 // product happens in registers, and a pass of two S-stage transforms needs
 // 2 S - 2 exchanges.  Inverse DFTs are forward ones of conjugates; the pointwise
 // functions conjugate.
 //
-// All constants that repeat in every slice (butterfly constants, stage twiddles,
-// chirps) are applied as float hi + lo parts, as in wap_fft.cuh.
+// All constants that repeat in every slice (butterfly constants, stage twiddles)
+// are applied as float hi + lo parts, as in wap_fft.cuh.
 #pragma once
 #include "wap_passes.cuh"
 
@@ -140,24 +138,17 @@ struct MixStep {
   float inv_L;
   const float2* src;   // buffer read, buffer written
   float2* dst;
-  bool load, end, last, chirp_turn;   // first stage of the pass; last of a transform; of the pass; turn by bhat
+  bool load, end, last;   // first stage of the pass; last of a transform; of the pass
 };
 
-template <int R, bool BLUE, class Op>
+template <int R, class Op>
 __device__ __forceinline__ void mix_butterfly(const GenAxis& ax, const MixStep& st, const float4* tw, int stride, int b,
                                               Op& op) {
   const int nb = ax.m / R;
   float2 v[R];
   if (st.load) {
 #pragma unroll
-    for (int j = 0; j < R; ++j) {
-      const int p = b + j * nb;
-      if (BLUE) {
-        v[j] = p < ax.n ? cmul_tw(op.load(p), __ldg(ax.chirp + p)) : make_float2(0.f, 0.f);
-      } else {
-        v[j] = op.load(p);
-      }
-    }
+    for (int j = 0; j < R; ++j) v[j] = op.load(b + j * nb);
   } else {
     const float2* s = st.src + b * stride;
     const int d = nb * stride;
@@ -175,28 +166,11 @@ __device__ __forceinline__ void mix_butterfly(const GenAxis& ax, const MixStep& 
   mix_dft<R>(v);
   int step = st.L;
   if (st.end) {
-    if (BLUE && !st.last && st.chirp_turn) {
 #pragma unroll
-      for (int j = 0; j < R; ++j) v[j] = cconj(cmul_tw(v[j], __ldg(ax.bhat + b + j * nb)));
-    } else {
-#pragma unroll
-      for (int j = 0; j < R; ++j) {
-        const int p = b + j * nb;
-        if (BLUE) {
-          float2 y = v[j];
-          v[j] = make_float2(0.f, 0.f);
-          if (p < ax.n) {
-            const float4 w = __ldg(ax.chirp + p);
-            y = cmul_tw(cconj(y), w);
-            if (st.last) op.store(p, y);
-            else v[j] = cmul_tw(op.turn(p, y), w);
-          }
-        } else if (st.last) {
-          op.store(p, v[j]);
-        } else {
-          v[j] = op.turn(p, v[j]);
-        }
-      }
+    for (int j = 0; j < R; ++j) {
+      const int p = b + j * nb;
+      if (st.last) op.store(p, v[j]);
+      else v[j] = op.turn(p, v[j]);
     }
     if (st.last) return;
     mix_dft<R>(v);
@@ -209,27 +183,16 @@ __device__ __forceinline__ void mix_butterfly(const GenAxis& ax, const MixStep& 
   for (int j = 0; j < R; ++j) o[j * d] = v[j];
 }
 
-template <int R, bool BLUE, class Op>
-__device__ __forceinline__ void mix_step(const GenAxis& ax, const MixStep& st, const float4* tw, int stride, int t,
-                                         Op& op) {
-  if (BLUE) {
-    for (int b = t; b * R < ax.m; b += ax.threads) mix_butterfly<R, true>(ax, st, tw, stride, b, op);
-  } else if (t * R < ax.m) {
-    mix_butterfly<R, false>(ax, st, tw, stride, t, op);
-  }
-}
-
 // `count` DFTs of the line (1 or 2): op.load(p) gives the input, op.turn(p, y) what
 // the second DFT takes in place of the first's result y, op.store(p, y) takes the
 // last one's result.  Every thread of the block calls it; `live` lines only do work.
-template <bool BLUE, class Op>
+template <class Op>
 __device__ __forceinline__ void mix_pass(const GenAxis& ax, int count, const float4* tw, const MixMem& mem, int t,
                                          bool live, Op& op) {
-  const int transforms = BLUE ? 2 * count : count;
   MixStep st;
   st.dst = mem.buf;
   st.src = mem.buf + mem.other;
-  for (int g = 0; g < transforms; ++g) {
+  for (int g = 0; g < count; ++g) {
     int L = 1;
     st.tw = (g & 1) ? ax.tw_rev : 0;
     for (int s = 0; s < ax.stages; ++s) {
@@ -238,11 +201,10 @@ __device__ __forceinline__ void mix_pass(const GenAxis& ax, int count, const flo
       st.inv_L = __fdividef(1.0f, (float)L);
       st.load = g == 0 && s == 0;
       st.end = s == ax.stages - 1;
-      st.last = st.end && g == transforms - 1;
-      st.chirp_turn = BLUE && !(g & 1);
+      st.last = st.end && g == count - 1;
       if (s > 0 || g == 0) {   // (later transforms' first stage belongs to the turn)
         if (live) switch (R) {
-#define WAP_MIX_CASE(r) case r: mix_step<r, BLUE>(ax, st, tw, mem.stride, t, op); break;
+#define WAP_MIX_CASE(r) case r: if (t * r < ax.m) mix_butterfly<r>(ax, st, tw, mem.stride, t, op); break;
           WAP_MIX_CASE(2) WAP_MIX_CASE(3) WAP_MIX_CASE(4) WAP_MIX_CASE(5) WAP_MIX_CASE(6) WAP_MIX_CASE(7)
           WAP_MIX_CASE(8)
 #undef WAP_MIX_CASE
