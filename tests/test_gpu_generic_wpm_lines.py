@@ -1,6 +1,8 @@
 """Wide-angle steps on grids that are not powers of two, by line kind: Bluestein
 lines of every transform length (64 .. 2048), both element counts per thread, one
-and several thread groups per row, beside mixed-radix and power-of-two sides.
+and several thread groups per row, beside mixed-radix and power-of-two sides; the
+fields of interpolation nodes and, on grids that reach the evanescent edge or
+with strong slices close to it, of the K reference indices.
 
 Bar: rel-L2 <= 1e-5 of exit wave, pattern and wavefronts against the FP64 oracle,
 as on the other paths.
@@ -45,3 +47,9 @@ SHAPES = [(31, 19, 1), (33, 37, 3), (64, 67, 2), (67, 100, 1), (97, 41, 5), (129
 @pytest.mark.parametrize("ny,nx,B", SHAPES)
 def test_nodes(wap, ny, nx, B):
     _check(wap, ny, nx, B, 6, 0.05)
+
+
+@pytest.mark.parametrize("ny,nx,B", SHAPES[:-1] + [(100, 60, 1), (45, 70, 3), (128, 100, 2), (30, 30, 40)])
+@pytest.mark.parametrize("ps,amp", [(0.01, 40.0), (0.01397, 600.0)])   # beyond the edge; short of it, strong slices
+def test_reference_fields(wap, ny, nx, B, ps, amp):
+    _check(wap, ny, nx, B, 3 if B > 100 else 7, ps, amp)

@@ -337,6 +337,7 @@ static void plan_free(wap_plan* p) {
   cudaFree(p->hvac_lo);
   cudaFree(p->ky2);
   cudaFree(p->kx2);
+  cudaFree(p->q);
   cudaFree(p->refs);
   cudaFree(p->slices);
   cudaFree(p->wn_tw_row);
@@ -408,6 +409,7 @@ int wap_plan_create(wap_plan** out, int ny, int nx, int max_batch, int op, int n
     if (err == cudaSuccess) err = cudaMalloc(&p->hvac_lo, plane * sizeof(float2));
     if (err == cudaSuccess) err = cudaMalloc(&p->ky2, ny * sizeof(float));
     if (err == cudaSuccess) err = cudaMalloc(&p->kx2, nx * sizeof(float));
+    if (err == cudaSuccess) err = cudaMalloc(&p->q, plane * sizeof(float));
     if (err != cudaSuccess) {
       plan_free(p);
       return cuda_fail(err, "cudaMalloc(WPM workspace)");

@@ -142,8 +142,8 @@ static cudaError_t launch_wcol_t(GenWpmColArgs& a, int nb, cudaStream_t st) {
   while (a.w > 4 && a.w * T > 32 && (long long)((nx + a.w - 1) / a.w) * nb < 296) a.w >>= 1;
   const size_t smem = FFTPlan<M, E>::TW_SIZE * sizeof(float4) + (size_t)(M + a.ax.n) * a.w * sizeof(float2);
   const int blocks = (nx + a.w - 1) / a.w;
-  return launch_gen(gen_wpm_col_kernel<BlueLine<M, E>>, dim3(blocks, nb, gen_wpm_shares(a, blocks, nb)), a.w * T, smem,
-                    st, a);
+  return launch_gen(a.refs ? gen_wpm_col_kernel<BlueLine<M, E>, true> : gen_wpm_col_kernel<BlueLine<M, E>, false>,
+                    dim3(blocks, nb, gen_wpm_shares(a, blocks, nb)), a.w * T, smem, st, a);
 }
 
 template <int M, int E>

@@ -33,8 +33,8 @@ static cudaError_t launch_gen_wcol(GenWpmColArgs& a, int nb, cudaStream_t st) {
   a.w = gen_cols(a.ax, c.nx, nb);
   const size_t smem = a.ax.tw_len * sizeof(float4) + 3 * (size_t)a.ax.m * a.w * sizeof(float2);
   const int blocks = (c.nx + a.w - 1) / a.w;
-  return launch_gen(gen_wpm_col_kernel<MixLine>, dim3(blocks, nb, gen_wpm_shares(a, blocks, nb)), a.w * a.ax.threads,
-                    smem, st, a);
+  return launch_gen(a.refs ? gen_wpm_col_kernel<MixLine, true> : gen_wpm_col_kernel<MixLine, false>,
+                    dim3(blocks, nb, gen_wpm_shares(a, blocks, nb)), a.w * a.ax.threads, smem, st, a);
 }
 
 static cudaError_t launch_gen_wrow(GenWpmRowArgs& a, int nb, cudaStream_t st) {
@@ -66,7 +66,7 @@ int generic_wpm_forward(const wap_plan* p, const WpmColArgs& cbase, const WpmRow
   r.ny = p->ny;
   r.nx = p->nx;
   r.flags = ROW_LOAD_SRC | ROW_FFT;
-  GenWpmColArgs c{wpm_node_col_args(p, cbase, nodes), p->gen_y, 0};
+  GenWpmColArgs c{wpm_node_col_args(p, cbase, nodes), p->gen_y, 0, !nodes.nodes};
   GenWpmRowArgs w{wpm_node_row_args(p, wbase, nodes, power), p->gen_x, inverse_scale(plane), 0, 0};
   for (int b0 = 0; b0 < n_probes; b0 += 65535) {
     const int nb = std::min(65535, n_probes - b0);

@@ -16,6 +16,7 @@ struct GenWpmColArgs {
   WpmNodeColArgs n;           // c.tw, c.kpg unused
   GenAxis ax;
   int w;                      // columns per block
+  bool refs;                  // every slice forms its reference fields
 };
 
 struct GenWpmSpectrum {       // column DFT -> spectrum * Hvac (* the centre node's factor), or the pattern
@@ -52,6 +53,7 @@ struct GenWpmSpectrum {       // column DFT -> spectrum * Hvac (* the centre nod
 struct GenWpmField {          // spectrum * the field's factor -> inverse column DFT
   const WpmNodeColArgs& na;
   const float2* hvac;
+  const float* q;             // this column's k0^2 - k_perp^2
   const float2* spec;
   float2* fcol;
   float2 ch, cl;              // the part taken off, propagated: added to every row
@@ -61,14 +63,14 @@ struct GenWpmField {          // spectrum * the field's factor -> inverse column
   __device__ __forceinline__ float2 load(int p) const {
     const WpmColArgs& a = na.c;
     float2 u = spec[p * w];
-    const float k2 = __ldg(a.ky2 + p) + kx2;
     if (nodes) {
       if (k > 0) {
+        const float k2 = __ldg(a.ky2 + p) + kx2;
         const float rest = wpm_slope_rest(a.k02 + a0 - k2, (na.dq - a0 + k2) * na.inv_qbar, na.kappa, na.inv_root_qbar);
         u = cmul(u, cism1(da * wpm_mean_slope(rest, na.kappa, da, a.dz, na.c4)));
       }
     } else {
-      const float q0 = a.k02 - k2, pr = 1.0f / q0, x = da * pr;
+      const float q0 = __ldg(q + p * a.nx), pr = 1.0f / q0, x = da * pr;
       if (q0 > 0.0f && fabsf(x) <= 0.0078125f)
         u = cmul(u, cis_small(da * (0.5f * a.dz * sqrtf(pr)) *
                               fmaf(x, fmaf(x, fmaf(x, -0.078125f, 0.125f), -0.25f), 1.0f)));
@@ -84,8 +86,9 @@ struct GenWpmField {          // spectrum * the field's factor -> inverse column
 };
 
 // Block group z forms the fields z, z + gridDim.z, ... (each repeats the forward
-// transform: a column pass of one probe is a few dozen blocks).
-template <class L>
+// transform: a column pass of one probe is a few dozen blocks).  REFS: the instance of
+// grids that reach the evanescent edge, where every slice forms its reference fields.
+template <class L, bool REFS>
 __global__ void __launch_bounds__(L::kCol, L::kColBlocks) gen_wpm_col_kernel(const GenWpmColArgs ga) {
   extern __shared__ float4 gen_smem[];
   const GenAxis& ax = ga.ax;
@@ -105,7 +108,7 @@ __global__ void __launch_bounds__(L::kCol, L::kColBlocks) gen_wpm_col_kernel(con
   const long long srow = (long long)d * a.n_slices + a.slice;
   const WpmSlice* rec = na.rec + srow;
   const int nf = rec->nf;
-  const bool nodes = rec->nodes != 0;
+  const bool nodes = !REFS && rec->nodes != 0;
 
   const auto mem = L::col_mem(ax, bufs, w, c);
   GenWpmSpectrum fwd{na};
@@ -130,6 +133,7 @@ __global__ void __launch_bounds__(L::kCol, L::kColBlocks) gen_wpm_col_kernel(con
   if (a.dp_mode) return;
   GenWpmField inv{na};
   inv.hvac = fwd.hvac;
+  inv.q = a.q + at;
   inv.spec = spec;
   inv.kx2 = fwd.kx2;
   inv.a0 = fwd.a0;

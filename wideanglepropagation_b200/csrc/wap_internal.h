@@ -54,6 +54,7 @@ struct wap_plan {
   float2* hvac_lo = nullptr;                // (ny, nx) lo part
   float* ky2 = nullptr;
   float* kx2 = nullptr;
+  float* q = nullptr;                       // (ny, nx) k0^2 - k_perp^2
   double hvac_key[4] = {0, 0, 0, 0};        // (dy, dx, dz, energy) of hvac
   float* refs = nullptr;                    // (draws, n_slices, n_bins)
   size_t refs_cap = 0;

@@ -595,6 +595,7 @@ struct WpmColArgs {
   const float2* hvac_lo;     // (ny, nx)  and lo part of the float64 value
   const float* ky2;          // (ny) (2 pi fy)^2
   const float* kx2;          // (nx) (2 pi fx)^2
+  const float* q;            // (ny, nx) k0^2 - k_perp^2
   const float* refs;         // (draws, n_slices, K)
   const int* draw;
   const float4* tw;
@@ -653,11 +654,10 @@ wpm_col_kernel(const WpmColArgs a) {
 
   // per element: q0 = k0^2 - k_perp^2, X * Hvac
   float q0[E];
-  const float kx2 = __ldg(a.kx2 + col);
 #pragma unroll
   for (int e = 0; e < E; ++e) {
     const int ky = t + T * e;
-    q0[e] = a.k02 - (__ldg(a.ky2 + ky) + kx2);
+    q0[e] = __ldg(a.q + (long long)ky * nx + col);
     v[e] = cmul_hl(v[e], __ldg(a.hvac + (long long)ky * nx + col), __ldg(a.hvac_lo + (long long)ky * nx + col));
   }
   // Bin phase dz a_k / (sqrt(q0 + a_k) + sqrt(q0)) = (dz a_k / (2 sqrt(q0))) f(a_k / q0)

@@ -25,7 +25,10 @@ namespace wap {
 
 // WPM vacuum propagator exp(i dz sqrt_c(k0^2 - k_perp^2)) in float64 on the
 // 'xy' meshgrid of propagation.py:224-228 (rows: ky = 2 pi fftfreq(ny, dy)),
-// rounded once to complex64, plus the float32 tables (2 pi f)^2 per axis.
+// rounded once to complex64, plus the float32 tables (2 pi f)^2 per axis and
+// q = k0^2 - k_perp^2.  q is rounded once: near the evanescent edge the difference
+// of the rounded terms (k0^2 is some 1e5) was off by as much as q, which put 2e-5
+// into the exit wave of a 64 x 67 grid with a mode there.
 struct HvacArgs {
   int ny, nx;
   double dy, dx, dz, k0;
@@ -33,6 +36,7 @@ struct HvacArgs {
   float2* hvac_lo;
   float* ky2;
   float* kx2;
+  float* q;
 };
 
 __global__ void wpm_vacuum_kernel(const HvacArgs a) {
@@ -50,6 +54,7 @@ __global__ void wpm_vacuum_kernel(const HvacArgs a) {
     im = 0.0;
   }
   const float rh = (float)re, ih = (float)im;
+  a.q[idx] = (float)q;
   a.hvac[idx] = make_float2(rh, ih);
   a.hvac_lo[idx] = make_float2((float)(re - (double)rh), (float)(im - (double)ih));
   if (ix == 0) a.ky2[iy] = (float)(ky * ky);
@@ -514,7 +519,7 @@ extern "C" int wap_wpm_fwd(wap_plan* p, const float* V, int n_slices, int n_draw
 
   const double key[4] = {sampling_y, sampling_x, dz, energy};
   if (!std::equal(key, key + 4, p->hvac_key)) {
-    HvacArgs h{p->ny, p->nx, sampling_y, sampling_x, dz, ph.k0, p->hvac, p->hvac_lo, p->ky2, p->kx2};
+    HvacArgs h{p->ny, p->nx, sampling_y, sampling_x, dz, ph.k0, p->hvac, p->hvac_lo, p->ky2, p->kx2, p->q};
     count_launch();
     wpm_vacuum_kernel<<<(unsigned)((plane + 255) / 256), 256, 0, st>>>(h);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "wpm_vacuum_kernel");
@@ -539,6 +544,7 @@ extern "C" int wap_wpm_fwd(wap_plan* p, const float* V, int n_slices, int n_draw
   c.hvac_lo = p->hvac_lo;
   c.ky2 = p->ky2;
   c.kx2 = p->kx2;
+  c.q = p->q;
   c.refs = p->refs;
   c.draw = draw;
   c.tw = p->tw_col;

@@ -183,10 +183,15 @@ wpm_node_col_kernel(const WpmNodeColArgs na) {
   // slope rest at q + a0 of this thread's elements (nodes; else q itself)
   const float kx2 = __ldg(a.kx2 + col);
   float p[E];
+  if (nodes) {
 #pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const float k2 = __ldg(a.ky2 + t + T * e) + kx2, q = a.k02 + a0 - k2;
-    p[e] = nodes ? wpm_slope_rest(q, (na.dq - a0 + k2) * na.inv_qbar, na.kappa, na.inv_root_qbar) : q;
+    for (int e = 0; e < E; ++e) {
+      const float k2 = __ldg(a.ky2 + t + T * e) + kx2;
+      p[e] = wpm_slope_rest(a.k02 + a0 - k2, (na.dq - a0 + k2) * na.inv_qbar, na.kappa, na.inv_root_qbar);
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < E; ++e) p[e] = __ldg(a.q + first + e * step);
   }
   __syncthreads();
   pdl_wait_then_release();
