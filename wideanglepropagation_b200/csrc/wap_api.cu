@@ -342,6 +342,7 @@ static void plan_free(wap_plan* p) {
   cudaFree(p->slices);
   cudaFree(p->wn_tw_row);
   cudaFree(p->wn_tw_col);
+  cudaFree(p->wn_tiles);
   cudaFree(p->ttab);
   for (void* d : p->kept) cudaFree(d);
   cudaFree(p->counter);

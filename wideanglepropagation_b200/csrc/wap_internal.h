@@ -62,6 +62,7 @@ struct wap_plan {
   size_t slices_cap = 0;
   float4* wn_tw_row = nullptr;              // (nx, 8) and (ny, 8) twiddles of the interpolating passes
   float4* wn_tw_col = nullptr;
+  unsigned* wn_tiles = nullptr;             // (batch, ny) finished shares of a row tile, zero between passes
   float2* ttab = nullptr;                   // transmission table (draws, n_slices, ny, nx)
   size_t ttab_cap = 0;
   // buffers that a captured call reads: kept when larger ones take their places, until the plan goes
@@ -135,6 +136,7 @@ int cluster_forward(wap_plan* p, const RowArgs& r, const ColArgs& c, int n_probe
 
 // reference values and interpolation records of every slice (wap_wpm.cu)
 struct WpmNodeScalars {
+  bool sharing = false;   // slices without nodes may be shared out to more blocks
   bool nodes = false;   // records may hold interpolation nodes (else every slice forms its K reference fields)
   // the slope dz / (2 sqrt(qbar)) taken out per pixel, and qbar - k0^2, 1 / qbar, 1 / sqrt(qbar)
   float kappa = 0.f, dq = 0.f, inv_qbar = 0.f, inv_root_qbar = 0.f;

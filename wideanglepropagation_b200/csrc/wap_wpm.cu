@@ -81,7 +81,7 @@ struct WpmSlicesArgs {
 // g (the variation of dz / (2 sqrt(q + a)) about kappa) and b_m the Taylor
 // coefficients of the square root, 2 theta |binom(1/2, m)| y^(m-1) with
 // theta = dz ah / (2 sqrt(q)) and y = ah / q at the smallest q.
-__device__ inline int wpm_node_count(double ah, double amax, double qmin, double k0, double dz, int most) {
+__host__ __device__ inline int wpm_node_count(double ah, double amax, double qmin, double k0, double dz, int most) {
   const double qe = qmin - amax - ah;
   const double y = ah / qe, th = fabs(dz) * ah / (2.0 * sqrt(qe));
   double g[kWpmMaxNodes + 1], e[kWpmMaxNodes + 1];
@@ -266,6 +266,24 @@ static cudaError_t node_smem(K kern, size_t smem) {
 // two 512^2 probes x 60 2.01 / 1.67 ms, one 1024^2 probe x 40 3.62 / 3.02 ms.
 static bool node_split(int n, long long lines) { return lines * (n / kNodeE) <= 148LL * 256; }
 
+// Blocks that share the K fields of a tile where a slice has no nodes: as many as the
+// chip holds beside the `ctas` of the pass (`per_sm` threads an SM), and at least two
+// fields for every group of each.
+static int node_shares(long long ctas, int threads, int per_sm, int K, int groups) {
+  return (int)std::max(1LL, std::min<long long>(148LL * per_sm / threads / ctas, K / (2 * groups)));
+}
+
+// Whether slices of a call may lack nodes with enough bins to share out (wpm_node_count
+// for an index whose square goes from 1 to 1 + kWpmIndexRange, 15 kV at 300 keV).  The
+// blocks that would share return from slices with nodes, but hold up the next pass's
+// early launch: 256^2, K = 128, 12.3 us a slice without them, 13.0 with.  Slices that
+// have no nodes take 234 us without them, 100 with.
+constexpr double kWpmIndexRange = 0.0625;
+static bool node_sharing(int K, double k0, double qmin, double dz) {
+  const double k02 = k0 * k0, amax = kWpmIndexRange * k02;
+  return K >= 16 && !(amax <= 0.125 * qmin && wpm_node_count(0.5 * amax, amax, qmin, k0, dz, kWpmMaxNodes) > 0);
+}
+
 template <int N, int G>
 static cudaError_t launch_node_col_t(const WpmNodeColArgs& a, int nb, cudaStream_t st) {
   constexpr int T = N / kNodeE;
@@ -275,14 +293,18 @@ static cudaError_t launch_node_col_t(const WpmNodeColArgs& a, int nb, cudaStream
   while (w > 1 && (w * T * G > node_col_threads(N, G) || w > a.c.nx)) w >>= 1;
   if (w == 8 && (long long)(a.c.nx / w) * nb < 148 && 4 * T >= 32) w = 4;
   const size_t smem = (size_t)N * w * G * sizeof(float2) + FFTPlan<N, kNodeE>::TW_SIZE * sizeof(float4);
-  cudaError_t e = node_smem(wpm_node_col_kernel<N, kNodeE, G>, smem);
+  const long long ctas = (long long)(a.c.nx / w) * nb;
+  const int per_sm = G > 1 || N >= 2048 ? 512 : 768;
+  const int z = a.sharing ? node_shares(ctas, w * T * G, per_sm, a.c.K, G) : 1;
+  auto kern = z > 1 ? wpm_node_col_kernel<N, kNodeE, G, true> : wpm_node_col_kernel<N, kNodeE, G, false>;
+  cudaError_t e = node_smem(kern, smem);
   if (e != cudaSuccess) return e;
   count_launch();
-  return launch_pdl(wpm_node_col_kernel<N, kNodeE, G>, dim3(a.c.nx / w, nb), w * T * G, smem, st, a);
+  return launch_pdl(kern, dim3(a.c.nx / w, nb, z), w * T * G, smem, st, a);
 }
 
 template <int N, int G>
-static cudaError_t launch_node_row_t(const WpmNodeRowArgs& a, int nb, cudaStream_t st) {
+static cudaError_t launch_node_row_t(WpmNodeRowArgs a, int nb, cudaStream_t st) {
   constexpr int T = N / kNodeE;
   // rows per CTA: kRowThreads threads per group (or half that with several
   // groups), fewer while SMs would be left without two CTAs; whole warps
@@ -292,10 +314,15 @@ static cudaError_t launch_node_row_t(const WpmNodeRowArgs& a, int nb, cudaStream
   // twiddles, pixel blends (28 bytes each), the groups' exchange segments, references
   const size_t smem = FFTPlan<N, kNodeE>::TW_SIZE * sizeof(float4) + (size_t)rows * N * 28 +
                       (size_t)rows * G * RowCfg<N, kNodeE>::PADN * sizeof(float2) + (size_t)a.r.K * sizeof(float);
-  cudaError_t e = node_smem(wpm_node_row_kernel<N, kNodeE, G>, smem);
+  const long long ctas = (long long)(a.r.ny / rows) * nb;
+  int z = a.sharing ? node_shares(ctas, rows * G * T, G > 1 ? 1024 : 768, a.r.K - 1, G) : 1;
+  a.r.kpg = (a.r.K - 2 + z) / z;
+  z = (a.r.K - 2 + a.r.kpg) / a.r.kpg;
+  auto kern = z > 1 ? wpm_node_row_kernel<N, kNodeE, G, true> : wpm_node_row_kernel<N, kNodeE, G, false>;
+  cudaError_t e = node_smem(kern, smem);
   if (e != cudaSuccess) return e;
   count_launch();
-  return launch_pdl(wpm_node_row_kernel<N, kNodeE, G>, dim3(a.r.ny / rows, nb), rows * G * T, smem, st, a);
+  return launch_pdl(kern, dim3(a.r.ny / rows, nb, z), rows * G * T, smem, st, a);
 }
 
 #define WAP_NODE_SIZES(M) M(32) M(64) M(128) M(256) M(512) M(1024) M(2048)
@@ -314,8 +341,12 @@ static cudaError_t launch_node_row(int n, const WpmNodeRowArgs& a, int nb, cudaS
   switch (n) { WAP_NODE_SIZES(WAP_NODE_ROW) default: return cudaErrorInvalidValue; }
 }
 
-// twiddles of the interpolating passes (plan creation)
+// twiddles and tile counts of the interpolating passes (plan creation)
 int wpm_node_twiddles(wap_plan* p) {
+  const size_t tiles = (size_t)p->ny * std::min(p->max_batch, 65535) * sizeof(unsigned);
+  cudaError_t err = cudaMalloc(&p->wn_tiles, tiles);
+  if (err == cudaSuccess) err = cudaMemset(p->wn_tiles, 0, tiles);
+  if (err != cudaSuccess) return cuda_fail(err, "WPM tile counts");
   for (int which = 0; which < 2; ++which) {
     float4*& d = which == 0 ? p->wn_tw_row : p->wn_tw_col;
     const std::vector<float4> h = twiddle_table(which == 0 ? p->nx : p->ny, kNodeE);
@@ -338,10 +369,11 @@ static double k2_max(int n, double d) {
 
 // Reference values and records of every slice.  Interpolation needs a grid that
 // stays clear of the evanescent edge (k0^2 above the largest k_perp^2).  Its passes
-// also serve the slices that then find no node count below K, with their K
-// reference fields: few bins, where they beat the split reference kernels (512^2,
-// K = 4: 0.83 against 1.84 ms for 40 slices); the evanescent grids keep those,
-// which share many bins out over more CTAs (256^2, K = 128: 1.7 against 4.1 ms for 20).
+// also serve the slices that then find no node count below K, with their K reference
+// fields: few bins, where they beat the split reference kernels (512^2, K = 4: 0.83
+// against 1.84 ms for 40 slices), and strong slices (node_sharing).  Where those fill
+// the chip they are the slower by up to a quarter (eight 256^2 probes, K = 32, 10
+// slices: 2.01 against 1.63 ms); the grids that reach the edge keep the reference kernels.
 static int wpm_slices(wap_plan* p, const float* V, int n_slices, int n_draws, const Physics& ph, double dz,
                       double sampling_y, double sampling_x, double power_spacing, WpmNodeScalars* out,
                       cudaStream_t st) {
@@ -375,6 +407,7 @@ static int wpm_slices(wap_plan* p, const float* V, int n_slices, int n_draws, co
     out->dq = (float)(qbar - ph.k0 * ph.k0);
     out->inv_qbar = (float)(1.0 / qbar);
     out->inv_root_qbar = (float)inv_root;
+    out->sharing = node_sharing(K, ph.k0, qmin, dz);
   }
   const long long plane = (long long)p->ny * p->nx;
   const WpmSlicesArgs a{V, p->refs, p->slices, (int)plane, n_slices, K, out->nodes ? 1 : 0, (float)ph.ri_a,
@@ -389,12 +422,12 @@ static int wpm_slices(wap_plan* p, const float* V, int n_slices, int n_draws, co
 
 WpmNodeColArgs wpm_node_col_args(const wap_plan* p, const WpmColArgs& c, const WpmNodeScalars& nodes) {
   WpmNodeColArgs n{c,          p->slices,      nodes.kappa,         nodes.dq, nodes.inv_qbar, nodes.inv_root_qbar,
-                   4.0f / (c.dz * c.dz)};
+                   4.0f / (c.dz * c.dz), nodes.sharing};
   n.c.tw = p->wn_tw_col;
   return n;
 }
 WpmNodeRowArgs wpm_node_row_args(const wap_plan* p, const WpmRowArgs& w, const WpmNodeScalars& nodes, double power) {
-  WpmNodeRowArgs n{w, p->slices, nodes.kk, power == 1.0 ? 1 : power == 2.0 ? 2 : 0};
+  WpmNodeRowArgs n{w, p->slices, p->wn_tiles, nodes.kk, power == 1.0 ? 1 : power == 2.0 ? 2 : 0, nodes.sharing};
   n.r.tw = p->wn_tw_row;
   return n;
 }
@@ -405,6 +438,7 @@ static int node_slices(const wap_plan* p, const WpmNodeScalars& nodes, const Wpm
   const long long plane = (long long)p->ny * p->nx;
   WpmNodeColArgs nc = wpm_node_col_args(p, c, nodes);
   WpmNodeRowArgs nr = wpm_node_row_args(p, w, nodes, power);
+  nr.r.blend = p->blend;
   cudaError_t e;
   for (int s = 0; s < n_slices; ++s) {
     nc.c.slice = nr.r.slice = s;

@@ -107,6 +107,7 @@ struct WpmNodeColArgs {
   float kappa;               // dz / (2 sqrt(qbar))
   float dq, inv_qbar, inv_root_qbar;   // qbar - k0^2, 1 / qbar, 1 / sqrt(qbar)
   float c4;                  // 4 / dz^2
+  bool sharing;              // launch only: slices without nodes may be shared out (SPLIT)
 };
 
 // Barrier of one group of threads of a block (whole warps).
@@ -150,7 +151,10 @@ __host__ __device__ constexpr int node_col_blocks(int n, int g) { return g > 1 |
 // for the whole column, is propagated beside it in float64 and added to the
 // results, row by row.  Drift of |psi| over 200 slices of 512^2, rms over
 // specimens: 5.9e-7 without, 4.1e-8 with (the exit wave's error 2.0e-6, 1.5e-6).
-template <int NY, int E, int G>
+//
+// SPLIT: a slice without nodes shares its K fields out to the blocks of grid.z too,
+// each of which repeats the forward part; a slice with nodes leaves them at once.
+template <int NY, int E, int G, bool SPLIT>
 __global__ void __launch_bounds__(node_col_threads(NY, G), node_col_blocks(NY, G))
 wpm_node_col_kernel(const WpmNodeColArgs na) {
   using P = FFTPlan<NY, E>;
@@ -173,14 +177,20 @@ wpm_node_col_kernel(const WpmNodeColArgs na) {
   const GroupColExchange xs{tiles + g * NY * W, W, c, 1 + g, group};
   // nothing here depends on the previous pass: twiddles and the slice's record
   // are read under its tail
-  for (int i = threadIdx.x; i < P::TW_SIZE; i += blockDim.x) tw[i] = __ldg(a.tw + i);
+  if constexpr (!SPLIT)
+    for (int i = threadIdx.x; i < P::TW_SIZE; i += blockDim.x) tw[i] = __ldg(a.tw + i);
   const int d = a.draw ? a.draw[b] : 0;
   const long long srow = (long long)d * a.n_slices + a.slice;
   const WpmSlice* rec = na.rec + srow;
+  if constexpr (SPLIT) {
+    if (blockIdx.z > 0 && rec->nodes) return;
+    for (int i = threadIdx.x; i < P::TW_SIZE; i += blockDim.x) tw[i] = __ldg(a.tw + i);
+  }
   const int nf = rec->nf;
   const bool nodes = rec->nodes != 0;
   const float a0 = rec->a0;   // 0 without nodes
-  // slope rest at q + a0 of this thread's elements (nodes; else q itself)
+  // slope rest at q + a0 of this thread's elements; without nodes the slope at q
+  // (0 beyond the evanescent edge)
   const float kx2 = __ldg(a.kx2 + col);
   float p[E];
   if (nodes) {
@@ -191,7 +201,10 @@ wpm_node_col_kernel(const WpmNodeColArgs na) {
     }
   } else {
 #pragma unroll
-    for (int e = 0; e < E; ++e) p[e] = __ldg(a.q + first + e * step);
+    for (int e = 0; e < E; ++e) {
+      const float q = __ldg(a.q + first + e * step);
+      p[e] = q > 0.0f ? 0.5f * a.dz * sqrtf(1.0f / q) : 0.0f;
+    }
   }
   __syncthreads();
   pdl_wait_then_release();
@@ -250,7 +263,8 @@ wpm_node_col_kernel(const WpmNodeColArgs na) {
   }
   float2* fcol = a.fields + (long long)b * a.K * plane + first;
   const float* refs = a.refs + srow * a.K;
-  for (int k = g; k < nf; k += G) {
+  const int shares = SPLIT && !nodes ? gridDim.z : 1;
+  for (int k = SPLIT ? blockIdx.z * G + g : g; k < nf; k += G * shares) {
     float2 u[E];
     if (nodes) {
       if (k == 0) {
@@ -266,12 +280,11 @@ wpm_node_col_kernel(const WpmNodeColArgs na) {
       const float ak = a.k02 * dk * (2.0f + dk);   // n_k^2 k0^2 - k0^2
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        const float pr = 1.0f / p[e], x = ak * pr;
-        if (p[e] > 0.0f && fabsf(x) <= 0.0078125f)
-          u[e] = cmul(v[e], cis_small(ak * (0.5f * a.dz * sqrtf(pr)) *
-                                      fmaf(x, fmaf(x, fmaf(x, -0.078125f, 0.125f), -0.25f), 1.0f)));
+        const float x = ak * na.c4 * p[e] * p[e];   // a_k / q
+        if (p[e] != 0.0f && fabsf(x) <= 0.0078125f)
+          u[e] = cmul(v[e], cis_small(ak * p[e] * fmaf(x, fmaf(x, fmaf(x, -0.078125f, 0.125f), -0.25f), 1.0f)));
         else
-          u[e] = wpm_bin_direct(v[e], pr, ak, a.dz, a.hvac + first + e * step);
+          u[e] = wpm_bin_direct(v[e], 1.0f / __ldg(a.q + first + e * step), ak, a.dz, a.hvac + first + e * step);
       }
     }
     fft<NY, E, true>(u, t, xs, tw);
@@ -354,10 +367,12 @@ __device__ __forceinline__ WpmPixel wpm_pixel(float volts, const float* srefs, i
 }
 
 struct WpmNodeRowArgs {
-  WpmRowArgs r;              // as the reference-field kernel (tw: the (nx, 8) table; no bin split)
+  WpmRowArgs r;              // as the reference-field kernel (tw: the (nx, 8) table; kpg: bins of a SPLIT share)
   const WpmSlice* rec;
+  unsigned* tiles;           // SPLIT: shares of each row tile that are done (zero between passes)
   float2 kk;                 // kappa k0^2, hi and lo parts
   int spacing;               // 1, 2: the references' power; 0: another
+  bool sharing;              // as WpmNodeColArgs::sharing
 };
 
 // Row exchange of one row of one group: its own segment, synchronised by the
@@ -382,7 +397,13 @@ struct GroupRowExchange {
 // shares through shared memory and goes on alone (as in the column pass).
 // The pixels' blends depend on the potential alone: the groups form them
 // together, before the wait for the column pass, and leave them in shared memory.
-template <int NX, int E, int G>
+//
+// SPLIT: a slice without nodes shares its bins out to the blocks of grid.z too, as in
+// wpm_row_kernel: block z owns the pixels whose left bin lies in [z kpg, z kpg + kpg),
+// passes over the bins that none of them wants, and stores their blend; the block of a
+// tile that is done last (a count per tile) takes the whole row on.  One 256^2 probe, K =
+// 128, 20 slices that have no nodes: 4.67 -> 2.01 ms (2.07 by the reference-field kernels).
+template <int NX, int E, int G, bool SPLIT>
 __global__ void __launch_bounds__(kRowThreads * (G > 1 ? 2 : 1), G > 1 ? 2 : 3)
 wpm_node_row_kernel(const WpmNodeRowArgs na) {
   using C = RowCfg<NX, E>;
@@ -406,6 +427,11 @@ wpm_node_row_kernel(const WpmNodeRowArgs na) {
   const int t = threadIdx.x & (T - 1);
   const int row = blockIdx.x * rows + rl;
   const int plane = a.ny * NX, at = row * NX + t;
+  if constexpr (SPLIT) {
+    if (blockIdx.z > 0 && (na.rec + srow)->nodes) return;
+  }
+  __shared__ unsigned used[SPLIT ? 128 : 1];   // bins (n_bins <= 4096) that this block's pixels want
+  __shared__ int last_share;
   const float* vrow = a.V + (long long)d * a.v_draw_stride + (long long)a.slice * plane + at;
   float vv[E / G];
 #pragma unroll
@@ -414,9 +440,13 @@ wpm_node_row_kernel(const WpmNodeRowArgs na) {
   for (int i = threadIdx.x; i < a.K; i += blockDim.x) srefs[i] = __ldg(a.refs + srow * a.K + i);
   for (int i = threadIdx.x; i < (int)(sizeof(WpmSlice) / 4); i += blockDim.x)
     reinterpret_cast<int*>(&srec)[i] = __ldg(reinterpret_cast<const int*>(na.rec + srow) + i);
+  if constexpr (SPLIT)
+    for (int i = threadIdx.x; i < 128; i += blockDim.x) used[i] = 0u;
   __syncthreads();
   const bool nodes = srec.nodes != 0;
   const int nf = srec.nf;
+  const bool split = SPLIT && !nodes;
+  const int kb = split ? blockIdx.z * a.kpg : 0, kl = split ? min(kb + a.kpg, a.K - 1) : 0;   // owned left bins
   spw += rl * NX;
   spt += rl * NX;
   sw += rl * NX;
@@ -427,6 +457,13 @@ wpm_node_row_kernel(const WpmNodeRowArgs na) {
     spw[x] = make_float4(px.pl.x, px.pl.y, px.pr.x, px.pr.y);
     spt[x] = make_float2(px.tl, px.tr);
     sw[x] = px.w;
+    if (SPLIT && split) {
+      const int il = __float_as_int(px.tl);
+      if (il >= kb && il < kl) {
+        atomicOr(used + (il >> 5), 1u << (il & 31));
+        atomicOr(used + ((il + 1) >> 5), 1u << ((il + 1) & 31));
+      }
+    }
   }
   __syncthreads();
   pdl_wait_then_release();
@@ -439,7 +476,10 @@ wpm_node_row_kernel(const WpmNodeRowArgs na) {
   for (int e = 0; e < E; ++e) acc[e] = make_float2(0.f, 0.f);
   const GroupRowExchange<T> xs{xbuf + (g * rows + rl) * C::PADN, 1 + g * rows + rl};
   const float2* frow = a.fields + (long long)b * a.K * plane + at;
-  for (int k = g < nf ? g + (nf - 1 - g) / G * G : -1; k >= 0; k -= G) {
+  const int n = split ? kl - kb + 1 : nf;   // fields of this block, from kb on
+  for (int i = g < n ? g + (n - 1 - g) / G * G : -1; i >= 0; i -= G) {
+    const int k = SPLIT ? kb + i : i;
+    if (SPLIT && split && !(used[k >> 5] & (1u << (k & 31)))) continue;
     const float2* fk = frow + (long long)k * plane;
 #pragma unroll
     for (int e = 0; e < E; ++e) u[e] = __ldcg(fk + T * e);
@@ -483,7 +523,7 @@ wpm_node_row_kernel(const WpmNodeRowArgs na) {
     }
     __syncthreads();
     if (g > 0) return;
-    const int shares = min(G, nf);
+    const int shares = min(G, n);
     for (int h = 1; h < shares; ++h) {
       const GroupRowExchange<T> xh{xbuf + (h * rows + rl) * C::PADN, 0};
 #pragma unroll
@@ -501,6 +541,27 @@ wpm_node_row_kernel(const WpmNodeRowArgs na) {
   }
 #pragma unroll
   for (int e = 0; e < E; ++e) acc[e] = cscale(acc[e], a.scale);
+
+  if (SPLIT && split && gridDim.z > 1) {
+    float2* brow = a.blend + (long long)b * plane + at;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int il = __float_as_int(spt[t + T * e].x);
+      if (il >= kb && il < kl) __stcg(brow + T * e, acc[e]);
+    }
+    __threadfence();
+    group_sync(15, group);   // (group 0 is what is left of the block)
+    if (threadIdx.x == 0) {
+      unsigned* done = na.tiles + (long long)blockIdx.y * gridDim.x + blockIdx.x;
+      last_share = atomicAdd(done, 1u) == gridDim.z - 1;
+      if (last_share) *done = 0u;
+      __threadfence();
+    }
+    group_sync(15, group);
+    if (!last_share) return;
+#pragma unroll
+    for (int e = 0; e < E; ++e) acc[e] = __ldcg(brow + T * e);
+  }
 
   if (a.snap) {
     float2* sp = a.snap + (long long)b * a.snap_bstride + at;
