@@ -24,8 +24,8 @@ import ctypes
 import threading
 
 from . import _lib
-from .propagation import (SCAN_GRAD_FROM_PROBES, SCAN_MIN_PROBES, StreamOrder, _detector, _device,  # noqa: F401
-                          _dp_shape, _prepare, _ptr, get_plan, scan_class, split_transfer)
+from .propagation import (SCAN_GRAD_FROM_PROBES, SCAN_MIN_PROBES, StreamOrder, _detector,  # noqa: F401
+                          _device, _dp_shape, _prepare, _ptr, get_plan, scan_class, split_transfer)
 
 # gradient scans (persistent scheduler) by shape, each with the StreamOrder of
 # its workspace; a scan is held from the forward until its backward has run,

@@ -449,7 +449,6 @@ def _prepare(potential, probe, positions, draw, dev):
     return V, psi, per_probe, pos, dr, B, n_slices, ny, nx, batched
 
 
-SCAN_MIN_PROBES = 8
 # Probes from which the persistent scheduler is the faster way on each grid: a step
 # of few small waves is a chain of hand-overs between its CTAs, 17 us a slice
 # whatever the count, where the pass kernels take 5 to 20.  Measured, 40 slices,
@@ -458,6 +457,8 @@ SCAN_MIN_PROBES = 8
 # 32 on 128^2 1.81 / 1.23, 16 on 256^2 1.98 / 1.86, 32 on 256^2 2.05 / 3.15.
 SCAN_FROM_PROBES = {128: 64, 256: 28, 512: 8, 1024: 8}
 SCAN_GRAD_FROM_PROBES = {128: 64, 256: 18, 512: 8, 1024: 8}
+# fewest probes that it takes on any grid
+SCAN_MIN_PROBES = min(*SCAN_FROM_PROBES.values(), *SCAN_GRAD_FROM_PROBES.values())
 # forwards of at most this many probes on these square grids may run as one launch (a
 # thread-block cluster per probe at 128, a cooperative grid where that is not to be had)
 CHAIN_SIZES = (128, 256)
