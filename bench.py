@@ -626,8 +626,9 @@ def baseline_table():
         ms = timeit(gpu, 20 if kind == "fresnel" else 5 if kind == "as" else 2)
         ex, dp, _ = gpu()
         npx = w.ny * w.nx
-        flops = w.n_slices * ((w.n_bins + 1) * 5.0 * npx * np.log2(npx) + 30.0 * w.n_bins * npx if kind == "wpm"
-                              else 10.0 * npx * np.log2(npx) + 24.0 * npx)
+        # one forward and one inverse transform and the factors of a slice: what any way of
+        # taking the step needs (a wide-angle one forms a few fields, whatever its bin count)
+        flops = w.n_slices * (10.0 * npx * np.log2(npx) + 24.0 * npx)
         t_bytes = 20.0 * npx * w.n_slices / (peak * 1e9)
         t_flops = flops / (fp32 * 1e12)
         rows[name] = {
