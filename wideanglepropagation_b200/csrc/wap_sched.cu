@@ -483,7 +483,28 @@ __device__ __forceinline__ void col_load(const float2* stage, float2 (&v)[E]) {
 }
 
 // Column tile: FFT, * H or conj(H) (hi + lo), [dp / adjoint seed], inverse FFT.
-template <int N, int E, bool GRAD, class TW>
+//
+// The exchange buffer between two tiles: the next tile may be published while compute
+// warps are still in this one, and a warp that has finished goes on with it.  Column
+// tiles, and row tiles of more than 32 threads a row, exchange across the whole block
+// and enter their first exchange through a block barrier, which a slow warp reaches
+// only with its last reads of the tile before done.  Row tiles of up to 32 threads a
+// row exchange within the warp and have no such barrier: their first store could
+// overwrite what a slow warp has yet to read (one call in sixty of 71 probes on 512^2,
+// 82 slices, had a wave spoilt).  So the warps meet once more, at the end of a
+// block-wide tile (END) or, where the tile count's top bit says that the last tile was
+// one, ahead of a warp-local one.  Measured, at the end / ahead: 1024 probes on 256^2
+// x 80 35.2 / 34.3 ms, 64 on 512^2 x 150 21.1 / 21.5, both sizes in one launch 54.4 /
+// 56.5 (its flag spills).
+template <unsigned MASK>
+__host__ __device__ constexpr bool meet_at_end() { return MASK != 1u && MASK != 2u; }
+constexpr uint32_t kBlockWide = 0x80000000u;
+__device__ __forceinline__ void meet_ahead(bool col, uint32_t& tiles_done) {
+  if (!col && (tiles_done & kBlockWide)) block_sync<kFftBar, kSchedThreads>();
+  tiles_done = col ? tiles_done | kBlockWide : tiles_done & ~kBlockWide;
+}
+
+template <int N, int E, bool GRAD, bool END, class TW>
 __device__ __forceinline__ void col_compute(const SchedClass& c, const Task& k, const Step& st, float2 (&v)[E],
                                             float2* exch, const TW* tw) {
   constexpr int T = N / E;
@@ -549,6 +570,7 @@ __device__ __forceinline__ void col_compute(const SchedClass& c, const Task& k, 
   float2* pcol = dst + (long long)k.b * plane + col;
 #pragma unroll
   for (int e = 0; e < E; ++e) __stcg(pcol + (long long)(t + T * e) * N, v[e]);
+  if constexpr (END) block_sync<kFftBar, kSchedThreads>();
 }
 
 // Compute warps of an instance for one grid size: take the published tile,
@@ -619,7 +641,8 @@ __device__ __forceinline__ void compute_loop_one(const SchedParams& P, float2* s
           __syncwarp();                                                     \
           if (lane == 0) mbar_arrive(empty);                                \
         }                                                                   \
-        if (col) col_compute<N, E, GRAD>(c, k, st, v, exch, tw);            \
+        if (!meet_at_end<MASK>()) meet_ahead(col, tiles_done);              \
+        if (col) col_compute<N, E, GRAD, meet_at_end<MASK>() && N / E <= 32>(c, k, st, v, exch, tw); \
         else row_compute<N, E, GRAD>(c, k, st, v, exch, tw, st2, acquire, release); \
       }                                                                     \
     }
@@ -724,8 +747,12 @@ __device__ __forceinline__ int tile_loop(const SchedParams& P, float2* stage, fl
       __syncwarp();
       if (lane == 0) mbar_arrive(empty);
     }
-    if (col) col_compute<N, E, GRAD>(c, k, st, v, exch, tw);
-    else row_compute<N, E, GRAD>(c, k, st, v, exch, tw, st2, acquire, release);
+    if (col) {
+      col_compute<N, E, GRAD, true>(c, k, st, v, exch, tw);
+    } else {
+      row_compute<N, E, GRAD>(c, k, st, v, exch, tw, st2, acquire, release);
+      if constexpr (N / E > 32) block_sync<kFftBar, kSchedThreads>();   // (another size's rows may follow)
+    }
     __syncwarp();
     if (lane == 0) mbar_arrive(done_bar + (cs.tiles_done & 1));
     ++cs.tiles_done;
