@@ -261,8 +261,8 @@ static cudaError_t node_smem(K kern, size_t smem) {
 
 // Whether a pass of `lines` lines of n points leaves the chip waiting on each
 // warp's chain of transforms, so that a line's fields go to several groups: up to
-// two one-group warps per scheduler.  Measured per call, K = 16, split / not: one
-// 512^2 probe x 200 slices 3.53 / 4.41 ms, four 256^2 probes x 100 1.55 / 2.07 ms;
+// two one-group warps per scheduler.  Measured per call, K = 16, split / not (when the
+// line was drawn): one 512^2 probe x 200 slices 3.53 / 4.41 ms, four 256^2 probes x 100 1.55 / 2.07 ms;
 // two 512^2 probes x 60 2.01 / 1.67 ms, one 1024^2 probe x 40 3.62 / 3.02 ms.
 static bool node_split(int n, long long lines) { return lines * (n / kNodeE) <= 148LL * 256; }
 

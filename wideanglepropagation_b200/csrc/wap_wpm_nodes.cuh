@@ -14,9 +14,9 @@
 // r is the smallest count whose remainder bound is below kWpmNodeTol for the
 // slice's range of a (wpm_node_count): 2 to 5 for light to heavy atoms, whatever K is.
 // The blend of the two bracketing references is unchanged, pixel by pixel; only
-// the K inverse transforms become r (one 512^2 probe, 200 slices, K = 16: 11.8 ->
-// 3.6 ms; 256^2, 40 slices, K = 128: 3.31 -> 0.47 ms).  A slice whose range has no such r < K, or
-// reaches towards the evanescent edge, forms its K reference fields as before
+// the K inverse transforms become r (one 512^2 probe, 200 slices, K = 16: 11.7 ->
+// 3.67 ms; 256^2, 40 slices, K = 128: 3.31 -> 0.47 ms).  A slice whose range has no
+// such r < K, or reaches towards the evanescent edge, forms its K reference fields
 // (nodes = 0 in its record).
 //
 // Fields are stored as the centre node's G_c and the differences G_j - G_c
