@@ -50,10 +50,25 @@ struct GenWpmSpectrum {       // column DFT -> spectrum * Hvac (* the centre nod
   }
 };
 
+// a reference field's factor on one element: the series of the column passes, or the
+// direct formulas near and beyond the edge
+__device__ __forceinline__ float2 gen_reference_value(float2 u, float q, float ak, float dz, const float2* hvac) {
+  const float pr = 1.0f / q, x = ak * pr;
+  if (q > 0.0f && fabsf(x) <= 0.0078125f)
+    return cmul(u, cis_small(ak * (0.5f * dz * sqrtf(pr)) *
+                             fmaf(x, fmaf(x, fmaf(x, -0.078125f, 0.125f), -0.25f), 1.0f)));
+  return wpm_bin_direct(u, pr, ak, dz, hvac);
+}
+// out of line in the instance whose slices mostly have nodes: one copy per kernel, not
+// one per radix, and no registers of theirs
+static __device__ __noinline__ float2 gen_reference_call(float2 u, float q, float ak, float dz, const float2* hvac) {
+  return gen_reference_value(u, q, ak, dz, hvac);
+}
+
+template <bool REFS>
 struct GenWpmField {          // spectrum * the field's factor -> inverse column DFT
   const WpmNodeColArgs& na;
   const float2* hvac;
-  const float* q;             // this column's k0^2 - k_perp^2
   const float2* spec;
   float2* fcol;
   float2 ch, cl;              // the part taken off, propagated: added to every row
@@ -70,12 +85,9 @@ struct GenWpmField {          // spectrum * the field's factor -> inverse column
         u = cmul(u, cism1(da * wpm_mean_slope(rest, na.kappa, da, a.dz, na.c4)));
       }
     } else {
-      const float q0 = __ldg(q + p * a.nx), pr = 1.0f / q0, x = da * pr;
-      if (q0 > 0.0f && fabsf(x) <= 0.0078125f)
-        u = cmul(u, cis_small(da * (0.5f * a.dz * sqrtf(pr)) *
-                              fmaf(x, fmaf(x, fmaf(x, -0.078125f, 0.125f), -0.25f), 1.0f)));
-      else
-        u = wpm_bin_direct(u, pr, da, a.dz, hvac + p * a.nx);
+      const float2* h = hvac + p * a.nx;
+      const float q = __ldg(a.q + (h - a.hvac));
+      u = REFS ? gen_reference_value(u, q, da, a.dz, h) : gen_reference_call(u, q, da, a.dz, h);
     }
     return cconj(u);
   }
@@ -131,9 +143,8 @@ __global__ void __launch_bounds__(L::kCol, L::kColBlocks) gen_wpm_col_kernel(con
   fwd.ref = apart ? __ldcg(a.psi + (long long)b * plane) : make_float2(0.f, 0.f);
   L::pass(ax, tw, mem, t, live, fwd);
   if (a.dp_mode) return;
-  GenWpmField inv{na};
+  GenWpmField<REFS> inv{na};
   inv.hvac = fwd.hvac;
-  inv.q = a.q + at;
   inv.spec = spec;
   inv.kx2 = fwd.kx2;
   inv.a0 = fwd.a0;
