@@ -31,6 +31,7 @@ int fail(int code, const char* fmt, ...) {
 }
 
 int cuda_fail(cudaError_t e, const char* what) {
+  cudaGetLastError();   // the caller has it now; the next call's launches do not see it again
   return fail(WAP_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
@@ -81,8 +82,8 @@ std::vector<float4> twiddle_table(int n, int e) {
 // ----------------------------------------------------------------------------
 template <class K>
 static cudaError_t prep_smem(K kern, size_t smem) {
-  if (smem > 48 * 1024) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  return cudaSuccess;
+  if (!beyond_default_smem(smem)) return cudaSuccess;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
 template <int N, int E>

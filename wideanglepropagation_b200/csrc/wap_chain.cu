@@ -125,8 +125,8 @@ static cudaError_t chain_launch_t(const ChainArgs& a, cudaStream_t st, int* grid
   auto kern = chain_kernel<N, E>;
   const size_t smem = chain_smem_bytes<N, E>();
   cudaError_t e;
-  if (smem > 48 * 1024 && (e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-                              cudaSuccess)
+  if (beyond_default_smem(smem) &&
+      (e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
     return e;
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);

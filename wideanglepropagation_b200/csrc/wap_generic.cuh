@@ -176,7 +176,7 @@ constexpr size_t kGenSmem = 200 * 1024;
 template <class K, class A>
 inline cudaError_t launch_gen(K kern, dim3 grid, int threads, size_t smem, cudaStream_t st, const A& a) {
   cudaError_t e;
-  if (smem > 48 * 1024 &&
+  if (beyond_default_smem(smem) &&
       (e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
     return e;
   count_launch();

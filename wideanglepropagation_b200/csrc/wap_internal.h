@@ -108,6 +108,9 @@ int stream_capture(cudaStream_t st);
 // gives up a buffer that a plan has outgrown: freed, or kept with the plan where a
 // captured call holds its address
 void drop_outgrown(wap_plan* p, void* d, bool captured);
+// whether a kernel has to be allowed this much dynamic shared memory: 48 KB is the
+// limit of dynamic and static together, and no kernel has 4 KB of static
+inline bool beyond_default_smem(size_t dynamic) { return dynamic > 44 * 1024; }
 int rows_per_cta(int nx, int e, int ny, int nb);
 bool size_supported(int n);
 

@@ -255,8 +255,9 @@ constexpr int kNodeE = 8;
 
 template <class K>
 static cudaError_t node_smem(K kern, size_t smem) {
-  return smem > 48 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                          : cudaSuccess;
+  return beyond_default_smem(smem)
+             ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+             : cudaSuccess;
 }
 
 // Whether a pass of `lines` lines of n points leaves the chip waiting on each
