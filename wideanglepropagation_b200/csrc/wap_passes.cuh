@@ -533,8 +533,9 @@ static __device__ __noinline__ float2 wpm_bin_direct(float2 v, float pr, float a
     return cmul(v, make_float2(c, s));
   }
   if (q0 < 0.0f && qk < 0.0f) return cscale(v, expf(dz * ak / (sqrtf(-qk) + sq0)));
-  // one side evanescent: exact H_k; undo the vacuum factor on X.  v = X * hv;
-  // |hv| is 1 (propagating vacuum) or a decay factor: divide it out explicitly
+  // one side evanescent: exact H_k; undo the vacuum factor on X.  v = X * hv with hv a
+  // phase (propagating vacuum) or a real decay, which is divided out (by its square it
+  // underflowed from a decay of 1e-19 on: modes lost, or NaN)
   const float2 hv = __ldg(hvac);
   float2 hk;
   if (qk >= 0.0f) {
@@ -544,8 +545,8 @@ static __device__ __noinline__ float2 wpm_bin_direct(float2 v, float pr, float a
   } else {
     hk = make_float2(expf(-dz * sqrtf(-qk)), 0.0f);
   }
-  const float n2 = fmaf(hv.x, hv.x, hv.y * hv.y);
-  const float2 x = n2 > 0.0f ? cscale(cmulc(v, hv), 1.0f / n2) : make_float2(0.f, 0.f);
+  float2 x = cmulc(v, hv);
+  if (q0 < 0.0f) x = hv.x >= 1.17549435e-38f ? make_float2(v.x / hv.x, v.y / hv.x) : make_float2(0.f, 0.f);
   return cmul(x, hk);
 }
 
